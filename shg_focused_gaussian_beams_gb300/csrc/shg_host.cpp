@@ -1868,7 +1868,7 @@ int shg_check_status(int *enabled, int *site, long long *value) {
     unsigned long long first = 0;
     for (auto take : {check_word_take_march, check_word_take_resident64, check_word_take_resident128,
                       check_word_take_resident256, check_word_take_cluster_pt, check_word_take_thermal,
-                      check_word_take_heat_tma, check_word_take_adjoint}) {
+                      check_word_take_heat_tma, check_word_take_heat_block, check_word_take_adjoint}) {
         const unsigned long long w = take();
         if (w == ~0ull) {
             set_error("shg_check_status: status word unreadable");

@@ -40,6 +40,7 @@ unsigned long long check_word_take_resident256();
 unsigned long long check_word_take_cluster_pt();
 unsigned long long check_word_take_thermal();
 unsigned long long check_word_take_heat_tma();
+unsigned long long check_word_take_heat_block();
 unsigned long long check_word_take_adjoint();
 cudaError_t launch_check_selftest(long long value);
 
@@ -86,15 +87,15 @@ cudaError_t launch_init_temperature(float *T, int nx, int ny, int nz, float temp
 // bounded pipeline waits gives up (read and cleared with heat_tma_error).
 cudaError_t launch_heat(float *Tf, const float *Ti, const float *QK, const HeatCoef &c, int nx, int ny, int nz,
                         int bc, int *err, cudaStream_t st);
-// K = levels sweeps in one launch (temporal blocking), levels in {2, 3, 4}; bit-identical
-// to K launch_heat calls. heat_levels(): the level count in use (SHG_HEAT_TB, default 1 =
-// no temporal blocking: the sweep is issue-bound, and the blocked form's redundant halo
-// updates cost more issue slots than its saved DRAM traffic on GB300).
-cudaError_t launch_heat_tb(float *Tf, const float *Ti, const float *QK, const HeatCoef &c, int nx, int ny, int nz,
-                           int bc, int levels, cudaStream_t st);
-int heat_levels();
-cudaError_t verify_fast_division(float d, float r, unsigned long long *d_count, unsigned long long *mismatches,
-                                 cudaStream_t st);
+cudaError_t verify_fast_division(float d, float r, unsigned long long *d_count, cudaStream_t st);
+// shg_heat_block.cu: one or two sweeps in one launch (NX % 4 == 0, 16-byte aligned buffers),
+// bit-identical to launch_heat calls. heat_block_plan chooses the tiling, and the sweeps per
+// launch where levels is 0.
+struct HeatBlockPlan;
+bool heat_block_supported(int nx, int ny, int nz);
+cudaError_t heat_block_plan(int nx, int ny, int nz, int bc, int levels, HeatBlockPlan *out);
+cudaError_t launch_heat_block(float *Tf, const float *Ti, const float *QK, const HeatCoef &c, int bc,
+                              const HeatBlockPlan &p, cudaStream_t st);
 // shg_heat_tma.cu: the TMA-staged sweep (NX % 4 == 0) and its pipeline error word. Each
 // THERMAL solve owns one device int; component calls lease one from a pool.
 bool heat_tma_supported(int nx, int ny, int nz);

@@ -16,6 +16,7 @@ struct HeatCoef {
     float den_x, den_y, den_z;   // 1 + 2a + 2b + Bi of the three face families
     float tinf;
     double KV, KH, KD;           // 0.5*T_inf*(Bix+Biz), 0.5*T_inf*(Biy+Biz), 0.5*T_inf*(Bix+Biy)
+    float KVh, KVl, KHh, KHl, KDh, KDl;  // each as the sum of two floats (edge_round)
     float tinfBix, tinfBiy, tinfBiz, tinfBiD;
     // Division of the interior stencil by dx^2, dy^2, dz^2: when fast_div is set, a / d is
     // formed as q = a*r, q + (a - q*d)*r with r = 1/d rounded, which was checked against
@@ -23,9 +24,25 @@ struct HeatCoef {
     // (verify_fast_division); other numerators use IEEE division.
     float rdx2, rdy2, rdz2;
     int fast_div;
+    // the same for the divisions of the face formulas by den_x, den_y, den_z
+    float rden_x, rden_y, rden_z;
+    int fast_face;
 };
 
 constexpr unsigned kDivExpLo = 27, kDivExpHi = 227;  // |a| in [2^-100, 2^101)
+
+// Tiling of one blocked heat launch (shg_heat_block.cu): a tile's region is vx vectors of four
+// columns by 2 threads / vx rows, of which txi columns and tyi rows are stored (xh columns and
+// yh rows of halo before them), marching chunks of zc planes.
+struct HeatBlockGrid {
+    int nx, ny, nz, vx, txi, tyi, xh, yh, zc;
+};
+struct HeatBlockPlan {
+    HeatBlockGrid g;
+    dim3 grid;
+    int threads, levels;  // per block; sweeps per launch
+    size_t smem;
+};
 
 // Thermal extension of one solve.
 struct ThermDesc {
@@ -117,6 +134,24 @@ __device__ __forceinline__ float div_const(float a, float d, float r, int fast) 
     return __fdiv_rn(a, d);
 }
 
+// (float)(((double)s + K) * (double)D), the edge formulas' last step (Tfield.h:162-195), with
+// K = kh + kl to 48 bits. The sum and product are carried as pairs of floats, which is within
+// 2^-44 (|s| + |K|) |D| of the exact value, as the double result is; where the float roundings of both
+// ends of that interval agree, that float is the answer, else (one in a million, and infinities
+// and NaN) the doubles decide. About 15 float instructions against five FP64 ones at 1/64 rate:
+// on the faces' threads these were a third of a step of the open-top sweep.
+__device__ __forceinline__ float edge_round(float s, double K, float kh, float kl, float D) {
+    const float h = __fadd_rn(s, kh), t = __fsub_rn(h, s);
+    const float e = __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(h, t)), __fsub_rn(kh, t)), kl);  // s + kh + kl - h
+    const float p = __fmul_rn(h, D);
+    const float lo = __fmaf_rn(e, D, __fmaf_rn(h, D, -p));
+    const float d = __fmul_rn(__fmul_rn(__fadd_rn(fabsf(s), fabsf(kh)), fabsf(D)), 0x1p-44f);
+    const float a = __fadd_rn(p, __fadd_rn(lo, d)), b = __fadd_rn(p, __fsub_rn(lo, d));
+    float r = a;
+    if (!(a == b)) r = __double2float_rn(__dmul_rn(__dadd_rn((double)s, K), (double)D));
+    return r;
+}
+
 // One voxel of Tfield.h:113-258 from its six face neighbours (only those the formula of
 // the voxel's class uses are read): xm/xp, ym/yp, zm/zp = T at x-1/x+1, y-1/y+1, z-1/z+1.
 // Returns false for voxels the reference never writes.
@@ -154,13 +189,13 @@ __device__ __forceinline__ bool heat_voxel(const HeatCoef &c, int x, int y, int 
         out = __fdiv_rn(s, c.den_y);
     } else if (xe && yi && ze) {
         const float s = __fadd_rn(__fadd_rn(__fmul_rn(c.av, txn), __fmul_rn(c.bv, tzn)), __fmul_rn(c.cv, __fadd_rn(yp, ym)));
-        out = __double2float_rn(__dmul_rn(__dadd_rn((double)s, c.KV), (double)c.V));
+        out = edge_round(s, c.KV, c.KVh, c.KVl, c.V);
     } else if (ytop && xi && ze) {
         const float s = __fadd_rn(__fadd_rn(__fmul_rn(c.ah, ym), __fmul_rn(c.bh, tzn)), __fmul_rn(c.ch, __fadd_rn(xm, xp)));
-        out = __double2float_rn(__dmul_rn(__dadd_rn((double)s, c.KH), (double)c.H));
+        out = edge_round(s, c.KH, c.KHh, c.KHl, c.H);
     } else if (xe && ytop && zi) {
         const float s = __fadd_rn(__fadd_rn(__fmul_rn(c.ad, ym), __fmul_rn(c.bd, txn)), __fmul_rn(c.cd, __fadd_rn(zp, zm)));
-        out = __double2float_rn(__dmul_rn(__dadd_rn((double)s, c.KD), (double)c.D));
+        out = edge_round(s, c.KD, c.KDh, c.KDl, c.D);
     } else if (xe && ytop && ze) {
         float s = __fadd_rn(__fmul_rn(c.AV, txn), __fmul_rn(c.BV, ym));
         s = __fadd_rn(s, __fmul_rn(c.CV, tzn));

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <cstdlib>
 #include <map>
@@ -76,6 +77,13 @@ HeatCoef make_heat_coef(const shg_config &cfg, float T_inf) {
     c.KV = 0.5 * (double)T_inf * (double)(c.Bix + c.Biz);
     c.KH = 0.5 * (double)T_inf * (double)(c.Biy + c.Biz);
     c.KD = 0.5 * (double)T_inf * (double)(c.Bix + c.Biy);
+    auto split = [](double k, float &hi, float &lo) {
+        hi = (float)k;
+        lo = (float)(k - (double)hi);
+    };
+    split(c.KV, c.KVh, c.KVl);
+    split(c.KH, c.KHh, c.KHl);
+    split(c.KD, c.KDh, c.KDl);
     c.tinfBix = c.Bix * T_inf;
     c.tinfBiy = c.Biy * T_inf;
     c.tinfBiz = c.Biz * T_inf;
@@ -87,30 +95,76 @@ int enable_fast_division(HeatCoef &c, cudaStream_t st) {
     static std::mutex mu;
     static std::map<std::pair<int, unsigned>, bool> verified;  // (device, divisor bits) -> exact
     static std::map<int, unsigned long long *> counters;
+    constexpr int kDivs = 6;
+    const float divs[kDivs] = {c.dx2, c.dy2, c.dz2, c.den_x, c.den_y, c.den_z};
     c.rdx2 = 1.0f / c.dx2;
     c.rdy2 = 1.0f / c.dy2;
     c.rdz2 = 1.0f / c.dz2;
-    c.fast_div = 0;
+    c.rden_x = 1.0f / c.den_x;
+    c.rden_y = 1.0f / c.den_y;
+    c.rden_z = 1.0f / c.den_z;
+    c.fast_div = c.fast_face = 0;
     if (std::getenv("SHG_HEAT_DIV") && std::string(std::getenv("SHG_HEAT_DIV")) == "ieee") return SHG_OK;
     int dev = 0;
     TH_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(mu);
-    bool all = true;
-    for (float d : {c.dx2, c.dy2, c.dz2}) {
+    auto key = [&](float d) {
         unsigned bits;
         std::memcpy(&bits, &d, sizeof(bits));
-        auto key = std::make_pair(dev, bits);
-        auto it = verified.find(key);
-        if (it == verified.end()) {
-            unsigned long long *&cnt = counters[dev];
-            if (!cnt) TH_CUDA(cudaMalloc(&cnt, sizeof(unsigned long long)));
-            unsigned long long bad = 1;
-            TH_CUDA(verify_fast_division(d, 1.0f / d, cnt, &bad, st));
-            it = verified.emplace(key, bad == 0).first;
-        }
-        all = all && it->second;
+        return std::make_pair(dev, bits);
+    };
+    bool missing = false;
+    for (float d : divs) missing |= verified.find(key(d)) == verified.end();
+    if (missing) {  // all divisors of this geometry in one go, one read-back
+        unsigned long long *&cnt = counters[dev];
+        if (!cnt) TH_CUDA(cudaMalloc(&cnt, kDivs * sizeof(unsigned long long)));
+        unsigned long long bad[kDivs];
+        TH_CUDA(cudaMemsetAsync(cnt, 0, sizeof(bad), st));
+        for (int k = 0; k < kDivs; ++k) TH_CUDA(verify_fast_division(divs[k], 1.0f / divs[k], cnt + k, st));
+        TH_CUDA(cudaMemcpyAsync(bad, cnt, sizeof(bad), cudaMemcpyDeviceToHost, st));
+        TH_CUDA(cudaStreamSynchronize(st));
+        for (int k = 0; k < kDivs; ++k) verified[key(divs[k])] = bad[k] == 0;
     }
-    c.fast_div = all ? 1 : 0;
+    c.fast_div = verified[key(c.dx2)] && verified[key(c.dy2)] && verified[key(c.dz2)];
+    c.fast_face = verified[key(c.den_x)] && verified[key(c.den_y)] && verified[key(c.den_z)];
+    return SHG_OK;
+}
+
+// Sweeps per launch asked for by SHG_HEAT_TB: 1 (one launch of launch_heat per sweep), 2 (2..4:
+// shg_heat_block.cu with two), or 0 where it is unset (heat_block_plan chooses). SHG_HEAT alone
+// (a kernel by name) means 1.
+static int heat_levels_asked() {
+    const char *e = std::getenv("SHG_HEAT_TB");
+    if (!e) return std::getenv("SHG_HEAT") ? 1 : 0;
+    const int v = std::atoi(e);
+    return (v >= 2 && v <= 4) ? 2 : 1;
+}
+
+// `n` Jacobi sweeps on `st` between buf[0] and buf[1], starting from buf[cur], which is
+// updated to the buffer that holds the result. Grids whose rows are whole 16-byte vectors take
+// the blocked kernel (shg_heat_block.cu, one or two sweeps per launch); others, unaligned
+// buffers and a kernel selected by name take one launch of launch_heat per sweep. With
+// `as_single` the buffers end as after n launches of one sweep: the result in buf[n & 1] (from
+// cur = 0), the state before the last sweep in the other.
+static int heat_sweeps_enqueue(float *const (&buf)[2], int &cur, const float *qk, const HeatCoef &hc, int nx, int ny,
+                               int nz, int bc, int n, bool as_single, int *err, cudaStream_t st) {
+    const int asked = heat_levels_asked();
+    const bool aligned = ((reinterpret_cast<uintptr_t>(buf[0]) | reinterpret_cast<uintptr_t>(buf[1]) |
+                           reinterpret_cast<uintptr_t>(qk)) & 15) == 0;
+    if (n <= 0) return SHG_OK;
+    if (asked == 1 || !aligned || !heat_block_supported(nx, ny, nz)) {
+        for (; n > 0; --n, cur ^= 1) TH_CUDA(launch_heat(buf[cur ^ 1], buf[cur], qk, hc, nx, ny, nz, bc, err, st));
+        return SHG_OK;
+    }
+    HeatBlockPlan p;
+    TH_CUDA(heat_block_plan(nx, ny, nz, bc, asked, &p));
+    int pairs = p.levels == 2 ? (as_single ? n - 1 : n) / 2 : 0;
+    // one pair less where the launches' count has to have n's parity (a pair is one launch)
+    if (as_single && (pairs & 1)) --pairs;
+    for (int k = 0; k < pairs; ++k, cur ^= 1) TH_CUDA(launch_heat_block(buf[cur ^ 1], buf[cur], qk, hc, bc, p, st));
+    n -= 2 * pairs;
+    if (n > 0 && p.levels != 1) TH_CUDA(heat_block_plan(nx, ny, nz, bc, 1, &p));
+    for (; n > 0; --n, cur ^= 1) TH_CUDA(launch_heat_block(buf[cur ^ 1], buf[cur], qk, hc, bc, p, st));
     return SHG_OK;
 }
 
@@ -193,16 +247,7 @@ int ThermalSolve::sweeps(float t_inf, int n) {
         TH_TRY(enable_fast_division(hc_, st_));
         tinf_coef_ = t_inf;
     }
-    const int L = heat_levels();
-    for (; L > 1 && n >= L; n -= L) {
-        TH_CUDA(launch_heat_tb(T_[cur_ ^ 1], T_[cur_], qk_, hc_, n_, n_, nz_, bc_, L, st_));
-        cur_ ^= 1;
-    }
-    for (int k = 0; k < n; ++k) {
-        TH_CUDA(launch_heat(T_[cur_ ^ 1], T_[cur_], qk_, hc_, n_, n_, nz_, bc_, err_, st_));
-        cur_ ^= 1;
-    }
-    return SHG_OK;
+    return heat_sweeps_enqueue(T_, cur_, qk_, hc_, n_, n_, nz_, bc_, n, false, err_, st_);
 }
 
 // A TMA-staged sweep whose pipeline gave up leaves its error word set: report it.
@@ -495,16 +540,10 @@ int shg_heat_sweeps_device(const shg_config *cfg, void *Ta, void *Tb, const void
         int *w;
         ~Lease() { heat_error_word_release(w); }
     } lease{err};
-    float *a = static_cast<float *>(Ta), *b = static_cast<float *>(Tb);
-    const int L = heat_levels();
-    for (; L > 1 && nsweeps >= L; nsweeps -= L) {
-        TH_CUDA(launch_heat_tb(b, a, static_cast<const float *>(QK), hc, cfg->nx, cfg->ny, cfg->nz, bc, L, st));
-        std::swap(a, b);
-    }
-    for (int k = 0; k < nsweeps; ++k) {
-        TH_CUDA(launch_heat(b, a, static_cast<const float *>(QK), hc, cfg->nx, cfg->ny, cfg->nz, bc, err, st));
-        std::swap(a, b);
-    }
+    float *const buf[2] = {static_cast<float *>(Ta), static_cast<float *>(Tb)};
+    int cur = 0;
+    TH_TRY(heat_sweeps_enqueue(buf, cur, static_cast<const float *>(QK), hc, cfg->nx, cfg->ny, cfg->nz, bc, nsweeps,
+                               true, err, st));
     // heat_pipeline_ok synchronises `st` and clears the word before it returns to the pool
     return heat_pipeline_ok(err, st);
 }
