@@ -7,7 +7,7 @@
 // delta-k(T) over slices 0..s (PhaseMatching.h:12-38), inc = 0, 0.25, 0.25, 0.5 per stage.
 // Both RK4 calls of step s use slice s. Per voxel the solve keeps a float4 table
 // (kp, ks, tpa1, DKint) built once from T; the stage constants are re-derived from it on
-// the fly (three sincosf per pixel and RK4 call).
+// the fly (th_coef_fixed).
 //
 // Batch layout: solve b owns states X + b*2*nn (pump then SH), tables coef + b*K*nn (slice
 // s at s*nn); one launch covers every solve (blockIdx.y = b).
@@ -35,7 +35,7 @@ __global__ void k_th_coef_table(const float *__restrict__ NP, const float *__res
 }
 
 __device__ __forceinline__ ThCoef th_coef_of(float4 cf, int s, float dz) {
-    return th_coef_k(cf.x, cf.y, cf.z, cf.w, s, dz);
+    return th_coef_fixed(cf.x, cf.y, cf.z, cf.w, s, dz);
 }
 
 // RK4_th^T of one point at the base state (P, S) with stage constants k: (cp, cs) hold the

@@ -442,14 +442,23 @@ struct ThRowShape {
     static_assert(FFT_THREADS % 32 == 0 && 2 * FFT_THREADS <= TPB, "transform threads fill whole warps");
 };
 
+// What a point of the persistent march keeps from one stage to the next: the coupling constants
+// and indices of the slice that its last RK4 call used, which the first call of the next stage
+// uses again, and the running delta-k sum.
+struct ThPoint {
+    ThCoef k;
+    float np, ns, dkint;
+};
+
 // The THERMAL row pass for lines [line0, line0 + LPB) at stage s on a block of
 // ThRowShape<N>::TPB threads (shared by the streaming launch and the persistent grid).
-// Twiddles: the global block g_twiddle + N, or with TS the split's pair table staged in
-// shared memory by the caller.
-template <int N, bool TS = false>
+// Twiddles: the global block g_twiddle + N, or, with KEEP (the persistent grid, whose blocks
+// hold at most one row unit), the split's pair table staged in shared memory by the caller;
+// KEEP also carries the point's constants in `pt` instead of forming them twice per slice.
+template <int N, bool KEEP = false>
 __device__ __forceinline__ void rows_th_body(const InstDesc &d, const ThermDesc &th, int line0, int s,
                                              float2 *scratch, float2 (*lines)[ThRowShape<N>::LPB * N],
-                                             const float2 *tab) {
+                                             const float2 *tab, ThPoint &pt) {
     using Sh = ThRowShape<N>;
     constexpr int G = Sh::G, E = N / G, LPB = Sh::LPB, FT = Sh::FFT_THREADS;
     constexpr int SC = LineScratch<N, G>::SIZE;
@@ -473,10 +482,12 @@ __device__ __forceinline__ void rows_th_body(const InstDesc &d, const ThermDesc 
     if (s == 0) {
         // DKint = DK(slice 0); RK4 of step 0; then the backward transform along x
         float2 vp = d.P[i2], vs = d.S[i2];
-        const float dkint = th.DK[i2];
-        th.DKint[i2] = dkint;
-        const ThCoef k = th_coef(th, th.NP[i2], th.NS[i2], dkint, 0, d.dz);
-        rk4_point_th(vp, vs, k, d);
+        pt.dkint = th.DK[i2];
+        pt.np = th.NP[i2];
+        pt.ns = th.NS[i2];
+        if (!KEEP) th.DKint[i2] = pt.dkint;
+        pt.k = th_coef(th, pt.np, pt.ns, pt.dkint, 0, d.dz);
+        rk4_point_th(vp, vs, pt.k, d);
         *pP = vp;
         *pS = vs;
         __syncthreads();
@@ -484,35 +495,40 @@ __device__ __forceinline__ void rows_th_body(const InstDesc &d, const ThermDesc 
             float2 v[E];
 #pragma unroll
             for (int j = 0; j < E; ++j) v[j] = fline[t + G * j];
-            fft_nat_to_spec<N, G, +1, false, 1, G + 1, TS>(v, t, fsc, tab);
+            fft_nat_to_spec<N, G, +1, false, 1, G + 1, KEEP>(v, t, fsc, tab);
 #pragma unroll
             for (int r = 0; r < E; ++r) F[fbase + spec_index<N, G>(t, r)] = v[r];
         }
         return;
     }
+    // the next slice's values first: their latency overlaps the transform
+    const size_t i3 = (size_t)(s - 1) * nxy + i2, i3n = (size_t)(s < th.nz ? s : s - 1) * nxy + i2;
+    const float npn = th.NP[i3n], nsn = th.NS[i3n], dkn = th.DK[i3n];
     // forward transform of the rows into natural x order
     if (xf) {
         float2 v[E];
 #pragma unroll
         for (int j = 0; j < E; ++j) v[j] = F[fbase + t + G * j];
-        fft_nat_to_spec<N, G, -1, false, 1, G + 1, TS>(v, t, fsc, tab);
+        fft_nat_to_spec<N, G, -1, false, 1, G + 1, KEEP>(v, t, fsc, tab);
 #pragma unroll
         for (int r = 0; r < E; ++r) fline[spec_index<N, G>(t, r)] = v[r];
+    }
+    if (!KEEP) {
+        pt.np = th.NP[i3];
+        pt.ns = th.NS[i3];
+        pt.dkint = th.DKint[i2];
+        pt.k = th_coef(th, pt.np, pt.ns, pt.dkint, s - 1, d.dz);
     }
     __syncthreads();
     const bool capture = (s == th.nz - 1);
     double aS = 0.0, aP = 0.0;
     {
         float2 vp = *pP, vs = *pS;
-        const size_t i3 = (size_t)(s - 1) * nxy + i2;
-        const float np1 = th.NP[i3], ns1 = th.NS[i3];
-        const float dkint = th.DKint[i2];
-        const ThCoef k1 = th_coef(th, np1, ns1, dkint, s - 1, d.dz);
-        rk4_point_th(vp, vs, k1, d);
+        rk4_point_th(vp, vs, pt.k, d);
         // Tfield.h:277-290: heat source of slice s-1 from the fields after step s-1
         const float a2p = fmaf(vp.x, vp.x, vp.y * vp.y);
         const float a2s = fmaf(vs.x, vs.x, vs.y * vs.y);
-        const float Ip = th.qc * np1 * a2p, Is = th.qc * ns1 * a2s;
+        const float Ip = th.qc * pt.np * a2p, Is = th.qc * pt.ns * a2s;
         const float Q = th.alpha_p * Ip + th.alpha_s * Is + th.beta_s * (Is * Is);
         SHG_AT(th.QK, i3, (size_t)th.nz * nxy, kChkThermalRows) = Q / th.kth;
         if (d.slices && s < th.nz) {
@@ -527,11 +543,12 @@ __device__ __forceinline__ void rows_th_body(const InstDesc &d, const ThermDesc 
             aP = (double)a2p;
         }
         if (s < th.nz) {
-            const size_t i3n = (size_t)s * nxy + i2;
-            const float dk2 = dkint + th.DK[i3n];
-            th.DKint[i2] = dk2;
-            const ThCoef k2 = th_coef(th, th.NP[i3n], th.NS[i3n], dk2, s, d.dz);
-            rk4_point_th(vp, vs, k2, d);
+            pt.np = npn;
+            pt.ns = nsn;
+            pt.dkint += dkn;
+            if (!KEEP) th.DKint[i2] = pt.dkint;
+            pt.k = th_coef(th, npn, nsn, pt.dkint, s, d.dz);
+            rk4_point_th(vp, vs, pt.k, d);
             *pP = vp;
             *pS = vs;
         } else {
@@ -550,7 +567,7 @@ __device__ __forceinline__ void rows_th_body(const InstDesc &d, const ThermDesc 
         float2 v[E];
 #pragma unroll
         for (int r = 0; r < E; ++r) v[r] = fline[spec_index<N, G>(t, r)];
-        fft_spec_to_nat<N, G, +1, false, 1, G + 1, TS>(v, t, fsc, tab);
+        fft_spec_to_nat<N, G, +1, false, 1, G + 1, KEEP>(v, t, fsc, tab);
 #pragma unroll
         for (int j = 0; j < E; ++j) F[fbase + t + G * j] = v[j];
     }
@@ -561,14 +578,16 @@ __global__ void __launch_bounds__(ThRowShape<N>::TPB) k_rows_th(const InstDesc *
     using Sh = ThRowShape<N>;
     __shared__ float2 scratch[2 * Sh::LPB * LineScratch<N, Sh::G>::SIZE];
     __shared__ float2 lines[2][Sh::LPB * N];  // [field][line * N + x], natural x order
-    rows_th_body<N>(*dd, th, blockIdx.x * Sh::LPB, s, scratch, lines, g_twiddle + N);
+    ThPoint pt;
+    rows_th_body<N>(*dd, th, blockIdx.x * Sh::LPB, s, scratch, lines, g_twiddle + N, pt);
 }
 
 // Persistent THERMAL march of one solve on a cooperative grid (stages 0..nz): the row pass
 // above and the plain column pass (cols_body_h, the same diffraction as k_cols) separated by
-// bounded grid-wide barriers instead of kernel boundaries. Block b runs row units b, b + B,
-// ... and column groups b + B w (warp w < col_warps), whose propagator values stay in
-// registers for the whole run. bar: zeroed arrival counter; err: the solve's error word, or-ed
+// bounded grid-wide barriers instead of kernel boundaries. The grid has at least one block per
+// row unit: block b runs row unit b, whose points' constants stay in registers from stage to
+// stage, and column groups b + B w (warp w < col_warps), whose propagator values stay there for
+// the whole run. bar: zeroed arrival counter; err: the solve's error word, or-ed
 // with 2 when a barrier wait gave up.
 template <int N>
 __global__ void __launch_bounds__(ThRowShape<N>::TPB) k_march_coop_th(const InstDesc *__restrict__ dd,
@@ -595,12 +614,11 @@ __global__ void __launch_bounds__(ThRowShape<N>::TPB) k_march_coop_th(const Inst
     const int f = u / (N / C::TC), x = (u % (N / C::TC)) * C::TC + lane % C::TC, t = lane / C::TC;
     float2 h[C::E];
     if (colw) hprop_load<N>(f == 0 ? d.Hp : d.Hs, x, t, h);
+    ThPoint pt;
     unsigned target = 0;
     for (int s = 0; s <= th.nz; ++s) {
-        for (int r = blockIdx.x; r < C::ROW_UNITS; r += gridDim.x) {
-            rows_th_body<N, true>(d, th, r * Sh::LPB, s, scratch, lines, tws);
-            __syncthreads();  // the block's line buffers are reused by its next unit
-        }
+        if (blockIdx.x < C::ROW_UNITS)
+            rows_th_body<N, true>(d, th, blockIdx.x * Sh::LPB, s, scratch, lines, tws, pt);
         if (s == th.nz) break;
         target += gridDim.x;
         if (!grid_barrier(bar, target, err, 2)) return;

@@ -64,8 +64,22 @@ struct ThCoef {
     float tpa1;
 };
 
+// sin and cos of a small angle by their Taylor series (truncated below 1e-9 for |x| <= 1/2),
+// sincosf beyond.
+__device__ __forceinline__ void sincos_small(float x, float &sn, float &cs) {
+    if (fabsf(x) <= 0.5f) {
+        const float y = x * x;
+        sn = fmaf(x * y, fmaf(y, fmaf(y, -1.0f / 5040.0f, 1.0f / 120.0f), -1.0f / 6.0f), x);
+        cs = fmaf(y, fmaf(y, fmaf(y, fmaf(y, 1.0f / 40320.0f, -1.0f / 720.0f), 1.0f / 24.0f), -0.5f), 1.0f);
+    } else {
+        sincosf(x, &sn, &cs);
+    }
+}
+
 // Stage constants from the per-pixel coupling factors kp = pi dQ / (n_p lp),
-// ks = 0.5 pi dQ / (n_s ls), the TPA factor and the running delta-k sum of slice s.
+// ks = 0.5 pi dQ / (n_s ls), the TPA factor and the running delta-k sum of slice s, with the
+// stage phases rounded as the THERMAL run has them: its heat source feeds back into T over five
+// outer iterations, which would spread another rounding.
 __device__ __forceinline__ ThCoef th_coef_k(float kp, float ks, float tpa1, float dkint, int s, float dz) {
     ThCoef r;
     const float sp1 = (float)(s + 1);
@@ -79,6 +93,28 @@ __device__ __forceinline__ ThCoef th_coef_k(float kp, float ks, float tpa1, floa
     sincosf(ph1, &sn, &cs);
     r.c1 = make_float4(kp * sn, kp * cs, -ks * sn, ks * cs);
     sincosf(ph2, &sn, &cs);
+    r.c2 = make_float4(kp * sn, kp * cs, -ks * sn, ks * cs);
+    r.tpa1 = tpa1;
+    return r;
+}
+
+// The same with the temperature field held fixed (the batched gradient): the phases are
+// DKint dz (1 + inc/(s+1)), so one sincosf at inc = 0 and two rotations by the angle
+// d = DKint dz / (4 (s+1)), a quarter step of the mean mismatch, serve the four stages. With
+// three sincosf and three divisions per RK4 call the constants were a third of the pointwise
+// passes: k_th_rk4_pair 25.4 -> 22.6 us, k_th_vjp_pair 36.5 -> 31.5 us at 16 x 256 x 256 points
+// (of which 14 us are the bytes that the first one moves, at HBM rate).
+__device__ __forceinline__ ThCoef th_coef_fixed(float kp, float ks, float tpa1, float dkint, int s, float dz) {
+    ThCoef r;
+    const float ph0 = dkint * dz, d = ph0 * __fdividef(0.25f, (float)(s + 1));
+    float sn, cs, sd, cd;
+    sincosf(ph0, &sn, &cs);
+    sincos_small(d, sd, cd);
+    r.c0 = make_float4(kp * sn, kp * cs, -ks * sn, ks * cs);
+    const float s1 = fmaf(sn, cd, cs * sd), c1 = fmaf(cs, cd, -sn * sd);
+    r.c1 = make_float4(kp * s1, kp * c1, -ks * s1, ks * c1);
+    sn = fmaf(s1, cd, c1 * sd);
+    cs = fmaf(c1, cd, -s1 * sd);
     r.c2 = make_float4(kp * sn, kp * cs, -ks * sn, ks * cs);
     r.tpa1 = tpa1;
     return r;
