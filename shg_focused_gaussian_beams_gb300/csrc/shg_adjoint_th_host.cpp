@@ -122,7 +122,7 @@ int ThermalGradBatch::setup_solve(int i, float power, float waist, float focal) 
     TG_CUDA(cudaMemcpyAsync(d_desc_ + i, &h_desc_[i], sizeof(InstDesc), cudaMemcpyHostToDevice, st));
     TG_CUDA(cudaMemsetAsync(h.acc, 0, 4 * sizeof(double), st));
     // Efields.h:74-126: Gaussian pump and shifted propagators at the centre temperature
-    TG_CUDA(launch_setup(d_desc_ + i, 1, (int)nn_, nz_, st));
+    TG_CUDA(launch_setup(d_desc_ + i, 1, (int)nn_, nz_, false, st));
     // loss scale: P_SH = 1/2 eps0 c n_s(tc) dx dy sum |S|^2 (the efficiency's convention)
     const float ns = crystal_index(cfg_.crystal, (float)(0.5 * (double)cfg_.lp), tc);
     const double seed = 2.0 * field_power(1.0, ns, h.dx, h.dy);

@@ -120,12 +120,12 @@ __global__ void __launch_bounds__(CptShape<N>::TPB, 1)
     for (int s = 0; s <= K; ++s) {
         // ---- row phase on the local rows (k_rows_pt's arithmetic)
         if (s == 0) {
-            const float4 c = d.stepc[0];
 #pragma unroll
             for (int k = 0; k < Sh::PTS; ++k) {
                 const int i = tid + Sh::TPB * k;
                 float2 p = sP[i], q = sS[i];
-                rk4_point(p, q, c, d);
+                march_enter(p, q, d);
+                rk4_march(p, q, d);
                 sP[i] = p;
                 sS[i] = q;
             }
@@ -156,19 +156,22 @@ __global__ void __launch_bounds__(CptShape<N>::TPB, 1)
             for (int k = 0; k < Sh::PTS; ++k) {
                 const int i = tid + Sh::TPB * k;
                 float2 p = sP[i], q = sS[i];
-                rk4_point(p, q, cprev, d);
+                rk4_march(p, q, d);
                 if (d.slices && s < d.nz) {
-                    float2 *sl = d.slices + (size_t)s * 2 * N * N;
-                    SHG_AT(sl, row0 + i, (size_t)2 * N * N, kChkSlices) = p;
-                    SHG_AT(sl, (size_t)N * N + row0 + i, (size_t)2 * N * N, kChkSlices) = q;
+                    float2 *sl = d.slices + (size_t)s * 2 * N * N, op = p, oq = q;
+                    march_leave(op, oq, cprev, d);
+                    SHG_AT(sl, row0 + i, (size_t)2 * N * N, kChkSlices) = op;
+                    SHG_AT(sl, (size_t)N * N + row0 + i, (size_t)2 * N * N, kChkSlices) = oq;
                 }
                 if (s == K) {
+                    march_leave(p, q, cprev, d);
                     SHG_AT(d.Pout, row0 + i, (size_t)N * N, kChkClusterPtRow) = p;
                     SHG_AT(d.Sout, row0 + i, (size_t)N * N, kChkClusterPtRow) = q;
                     aS += (double)q.x * q.x + (double)q.y * q.y;
                     aP += (double)p.x * p.x + (double)p.y * p.y;
                 } else {
-                    rk4_point(p, q, ccur, d);
+                    march_turn(q, ccur);
+                    rk4_march(p, q, d);
                     sP[i] = p;
                     sS[i] = q;
                 }

@@ -95,6 +95,18 @@ float crystal_index(int crystal, float L, float T) {
     return crystal == SHG_CRYSTAL_PPLN ? sellmeier_ln(L, T) : sellmeier(L, T);
 }
 
+// Scales of the marched fields (shg_march.cuh): they make both coupling constants of dA/dz equal
+// to 1. Without coupling (d_eff = 0, or so small that its square underflows) the fields are held
+// so small that the products vanish against them and p^2 underflows to zero.
+static void march_scales(InstDesc &d) {
+    const bool coupled = std::fabs(d.kp) >= 0x1p-60f && std::fabs(d.ks) >= 0x1p-60f;
+    d.ss = coupled ? d.kp : 0x1p-60f;
+    d.sp = coupled ? sqrtf(d.kp * d.ks) : 0x1p-100f;
+    d.isp = 1.0f / d.sp;
+    d.iss = 1.0f / d.ss;
+    d.tpa1s = (float)((double)d.tpa1 / ((double)d.ss * (double)d.ss));
+}
+
 // Fill the scalar part of a descriptor (pointers are set by the caller).
 void fill_scalars(const shg_config &cr, const SolveParams &sp, InstDesc &d) {
     const Phys ph;
@@ -117,6 +129,7 @@ void fill_scalars(const shg_config &cr, const SolveParams &sp, InstDesc &d) {
     d.hp = (float)(0.5 * (double)cr.alpha_p);
     d.tpa0 = (float)(0.5 * (double)cr.alpha_s);
     d.tpa1 = (float)(0.5 * ((double)cr.beta_s * 0.5 * (double)ph.C * (double)ph.EPS0 * (double)ns_t));
+    march_scales(d);
     // PhaseMatching.h:57-70
     d.dk = 2.0f * PI * (2.0f * np_t / lp - ns_t / ls + 1.0f / cr.lambda_qpm);
     // Efields.h:74-104 at tpump
@@ -557,7 +570,7 @@ class Batch {
                 for (int rep = 0; rep < 2 && rc == SHG_OK; ++rep) {
                     rc = enqueue_inputs(st);
                     if (rc) break;
-                    if (launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, st) != cudaSuccess ||
+                    if (launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, true, st) != cudaSuccess ||
                         cudaMemsetAsync(d_counters_, 0, 64 * sizeof(int), st) != cudaSuccess ||
                         cudaEventRecord(a, st) != cudaSuccess) {
                         rc = SHG_ERR_CUDA;
@@ -755,7 +768,7 @@ class Batch {
             desc_dirty_ = false;
         }
         SHG_TRY_INT(enqueue_inputs(st));
-        SHG_CUDA(launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, st));
+        SHG_CUDA(launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, true, st));
         SHG_CUDA(cudaMemsetAsync(d_counters_, 0, 64 * sizeof(int), st));
         const int nc = (int)classes_.size();
         std::vector<cudaEvent_t> ev(2 * nc + 1);
@@ -929,7 +942,7 @@ class Batch {
             desc_dirty_ = false;
         }
         SHG_TRY_INT(enqueue_inputs(st));
-        SHG_CUDA(launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, st));
+        SHG_CUDA(launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, false, st));
         return SHG_OK;
     }
 
@@ -960,7 +973,7 @@ class Batch {
                 SHG_CUDA(cudaMemsetAsync(desc_[i].S, 0, bytes, st));
         }
         if (rec) SHG_TRY_INT(rec->begin("setup", 24.0 * (double)total_points(), st));
-        SHG_CUDA(launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, st));
+        SHG_CUDA(launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, true, st));
         if (rec) SHG_TRY_INT(rec->end(st));
         for (int i = 0; i < (int)desc_.size(); ++i)
             if (desc_[i].slices) {

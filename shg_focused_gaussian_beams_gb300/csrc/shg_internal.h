@@ -58,7 +58,8 @@ cudaError_t launch_resident(int n, ResidentVariant v, const InstDesc *inst, cons
                             int max_clusters, cudaStream_t st);
 
 // shg_march.cu
-cudaError_t launch_setup(const InstDesc *inst, int n_inst, int max_nn, int max_nz, cudaStream_t st);
+// frame: stepc as the plain march reads it, else as the adjoint does (InstDesc).
+cudaError_t launch_setup(const InstDesc *inst, int n_inst, int max_nn, int max_nz, bool frame, cudaStream_t st);
 cudaError_t launch_rows(int n, const InstDesc *inst, const int *list, int count, int s, cudaStream_t st);
 cudaError_t launch_cols(int n, const InstDesc *inst, const int *list, int count, cudaStream_t st);
 // The whole march of one solve (list[0]) as one cooperative launch with bounded grid

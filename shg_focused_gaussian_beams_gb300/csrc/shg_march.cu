@@ -51,7 +51,8 @@ cudaError_t launch_check_selftest(long long value) {
 
 // z accumulates in float (Solver.h:271), one thread walks the slices of one solve; the
 // phase exp(-+ i z dk) enters dA/dz through cosf/sinf of fl(z*dk) (Operators.h:105-117).
-__global__ void k_setup_steps(const InstDesc *__restrict__ inst, int n_inst) {
+// frame: the march's constants (frames of consecutive slices), else the adjoint's.
+__global__ void k_setup_steps(const InstDesc *__restrict__ inst, int n_inst, int frame) {
     extern __shared__ float zs[];
     const InstDesc &d = inst[blockIdx.x];
     if (threadIdx.x == 0) {
@@ -66,7 +67,12 @@ __global__ void k_setup_steps(const InstDesc *__restrict__ inst, int n_inst) {
         const float arg = __fmul_rn(zs[s], d.dk);
         float sn, cs;
         sincosf(arg, &sn, &cs);
-        d.stepc[s] = make_float4(d.kp * sn, d.kp * cs, -d.ks * sn, d.ks * cs);
+        if (frame) {
+            const float turn = s > 0 ? __fsub_rn(arg, __fmul_rn(zs[s - 1], d.dk)) : 0.0f, h = sinf(0.5f * turn);
+            d.stepc[s] = make_float4(-2.0f * h * h, sinf(turn), cs, sn);
+        } else {
+            d.stepc[s] = make_float4(d.kp * sn, d.kp * cs, -d.ks * sn, d.ks * cs);
+        }
     }
 }
 
@@ -162,9 +168,11 @@ __global__ void __launch_bounds__(RowShape<N>::TPB) k_rows(const InstDesc *__res
         vs[j] = SHG_AT(d.S, base + t + G * j, NN, kChkRowsGlobal);
     }
     if (s == 0) {
-        const float4 c = d.stepc[0];
 #pragma unroll
-        for (int j = 0; j < E; ++j) rk4_point(vp[j], vs[j], c, d);
+        for (int j = 0; j < E; ++j) {
+            march_enter(vp[j], vs[j], d);
+            rk4_march(vp[j], vs[j], d);
+        }
         fft_nat_to_spec<N, G, +1>(vp, t, sc, tab);
         fft_nat_to_spec<N, G, +1>(vs, t, sc, tab);
 #pragma unroll
@@ -179,14 +187,16 @@ __global__ void __launch_bounds__(RowShape<N>::TPB) k_rows(const InstDesc *__res
     fft_nat_to_spec<N, G, -1>(vs, t, sc, tab);
     const float4 c1 = d.stepc[s - 1];
 #pragma unroll
-    for (int r = 0; r < E; ++r) rk4_point(vp[r], vs[r], c1, d);
+    for (int r = 0; r < E; ++r) rk4_march(vp[r], vs[r], d);
     if (d.slices && s < d.nz) {
         float2 *sl = d.slices + (size_t)s * 2 * N * N;
 #pragma unroll
         for (int r = 0; r < E; ++r) {
             const int k = spec_index<N, G>(t, r);
-            SHG_AT(sl, base + k, 2 * NN, kChkSlices) = vp[r];
-            SHG_AT(sl, NN + base + k, 2 * NN, kChkSlices) = vs[r];
+            float2 op = vp[r], os = vs[r];
+            march_leave(op, os, c1, d);
+            SHG_AT(sl, base + k, 2 * NN, kChkSlices) = op;
+            SHG_AT(sl, NN + base + k, 2 * NN, kChkSlices) = os;
         }
     }
     if (s == d.nsteps) {
@@ -194,6 +204,7 @@ __global__ void __launch_bounds__(RowShape<N>::TPB) k_rows(const InstDesc *__res
 #pragma unroll
         for (int r = 0; r < E; ++r) {
             const int k = spec_index<N, G>(t, r);
+            march_leave(vp[r], vs[r], c1, d);
             SHG_AT(d.Pout, base + k, NN, kChkRowsGlobal) = vp[r];
             SHG_AT(d.Sout, base + k, NN, kChkRowsGlobal) = vs[r];
             aS += (double)vs[r].x * vs[r].x + (double)vs[r].y * vs[r].y;
@@ -205,7 +216,10 @@ __global__ void __launch_bounds__(RowShape<N>::TPB) k_rows(const InstDesc *__res
     }
     const float4 c2 = d.stepc[s];
 #pragma unroll
-    for (int r = 0; r < E; ++r) rk4_point(vp[r], vs[r], c2, d);
+    for (int r = 0; r < E; ++r) {
+        march_turn(vs[r], c2);
+        rk4_march(vp[r], vs[r], d);
+    }
     fft_spec_to_nat<N, G, +1>(vp, t, sc, tab);
     fft_spec_to_nat<N, G, +1>(vs, t, sc, tab);
 #pragma unroll
@@ -256,7 +270,8 @@ __device__ __forceinline__ void rows_pt_body(const InstDesc &d, int line0, int s
 
     if (s == 0) {
         float2 vp = d.P[i2], vs = d.S[i2];
-        rk4_point(vp, vs, d.stepc[0], d);
+        march_enter(vp, vs, d);
+        rk4_march(vp, vs, d);
         *pP = vp;
         *pS = vs;
         __syncthreads();
@@ -270,6 +285,7 @@ __device__ __forceinline__ void rows_pt_body(const InstDesc &d, int line0, int s
         }
         return;
     }
+    const float4 turn = d.stepc[s];  // before the transform, which hides its latency (s <= nsteps < nz)
     if (xf) {
         float2 v[E];
 #pragma unroll
@@ -280,20 +296,24 @@ __device__ __forceinline__ void rows_pt_body(const InstDesc &d, int line0, int s
     }
     __syncthreads();
     float2 vp = *pP, vs = *pS;
-    rk4_point(vp, vs, d.stepc[s - 1], d);
+    rk4_march(vp, vs, d);
     if (d.slices && s < d.nz) {
         float2 *sl = d.slices + (size_t)s * 2 * N * N;
-        sl[i2] = vp;
-        sl[(size_t)N * N + i2] = vs;
+        float2 op = vp, os = vs;
+        march_leave(op, os, d.stepc[s - 1], d);
+        sl[i2] = op;
+        sl[(size_t)N * N + i2] = os;
     }
     if (s == d.nsteps) {
+        march_leave(vp, vs, d.stepc[s - 1], d);
         d.Pout[i2] = vp;
         d.Sout[i2] = vs;
         block_add_double((double)vs.x * vs.x + (double)vs.y * vs.y, d.acc + 1);
         block_add_double((double)vp.x * vp.x + (double)vp.y * vp.y, d.acc + 2);
         return;
     }
-    rk4_point(vp, vs, d.stepc[s], d);
+    march_turn(vs, turn);
+    rk4_march(vp, vs, d);
     *pP = vp;
     *pS = vs;
     __syncthreads();
@@ -594,9 +614,9 @@ cudaError_t launch_cols(int n, const InstDesc *inst, const int *list, int count,
     }
 }
 
-cudaError_t launch_setup(const InstDesc *inst, int n_inst, int max_nn, int max_nz, cudaStream_t st) {
+cudaError_t launch_setup(const InstDesc *inst, int n_inst, int max_nn, int max_nz, bool frame, cudaStream_t st) {
     if (n_inst <= 0) return cudaSuccess;
-    k_setup_steps<<<n_inst, 256, (size_t)max_nz * sizeof(float), st>>>(inst, n_inst);
+    k_setup_steps<<<n_inst, 256, (size_t)max_nz * sizeof(float), st>>>(inst, n_inst, frame);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     dim3 grid((max_nn + 1023) / 1024, n_inst);

@@ -156,7 +156,7 @@ extern "C" int shg_cwes_noalloc(const shg_config *cfg, float temp, const void *p
         NOALLOC_CUDA(cudaMemcpyAsync(d.S, sh_in, bytes, cudaMemcpyDeviceToDevice, st));
     else
         NOALLOC_CUDA(cudaMemsetAsync(d.S, 0, bytes, st));
-    NOALLOC_CUDA(launch_setup(d_desc, 1, n * n, cfg->nz, st));
+    NOALLOC_CUDA(launch_setup(d_desc, 1, n * n, cfg->nz, true, st));
     const int K = cfg->nz - 1;
     for (int s = 0; s <= K; ++s) {
         NOALLOC_CUDA(launch_rows(n, d_desc, d_list, 1, s, st));

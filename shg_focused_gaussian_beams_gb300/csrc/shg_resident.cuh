@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(ResShape<N, CS_, MINB_, G_>::THREADS, MINB_)
             // ---- row phase (local rows)
             {
                 float2 *rowP = sP + line * N, *rowS = sS + line * N;
-                // step constants of slices s-1 and s (s <= K < nz), loaded before the transform
+                // frames of slices s-1 and s (s <= K < nz), loaded before the transform
                 const float4 cprev = d.stepc[s > 0 ? s - 1 : 0], ccur = d.stepc[s];
                 float2 vp[E], vs[E];
 #pragma unroll
@@ -112,9 +112,11 @@ __global__ void __launch_bounds__(ResShape<N, CS_, MINB_, G_>::THREADS, MINB_)
                     vs[j] = rowS[t + G * j];
                 }
                 if (s == 0) {
-                    const float4 c = ccur;
 #pragma unroll
-                    for (int j = 0; j < E; ++j) rk4_point(vp[j], vs[j], c, d);
+                    for (int j = 0; j < E; ++j) {
+                        march_enter(vp[j], vs[j], d);
+                        rk4_march(vp[j], vs[j], d);
+                    }
                     fft_nat_to_spec<N, G, +1, false, 1, G + 1, true>(vp, t, rsc, tab);
                     fft_nat_to_spec<N, G, +1, false, 1, G + 1, true>(vs, t, rsc, tab);
                     __syncwarp();
@@ -127,17 +129,18 @@ __global__ void __launch_bounds__(ResShape<N, CS_, MINB_, G_>::THREADS, MINB_)
                 } else {
                     fft_nat_to_spec<N, G, -1, false, 1, G + 1, true>(vp, t, rsc, tab);
                     fft_nat_to_spec<N, G, -1, false, 1, G + 1, true>(vs, t, rsc, tab);
-                    const float4 c1 = cprev;
 #pragma unroll
-                    for (int r = 0; r < E; ++r) rk4_point(vp[r], vs[r], c1, d);
+                    for (int r = 0; r < E; ++r) rk4_march(vp[r], vs[r], d);
                     if (d.slices && s < d.nz) {
                         float2 *sl = d.slices + (size_t)s * 2 * N * N;
                         const size_t base = (size_t)(rank * R + line) * N;
 #pragma unroll
                         for (int r = 0; r < E; ++r) {
                             const int k = spec_index<N, G>(t, r);
-                            SHG_AT(sl, base + k, (size_t)2 * N * N, kChkSlices) = vp[r];
-                            SHG_AT(sl, (size_t)N * N + base + k, (size_t)2 * N * N, kChkSlices) = vs[r];
+                            float2 op = vp[r], os = vs[r];
+                            march_leave(op, os, cprev, d);
+                            SHG_AT(sl, base + k, (size_t)2 * N * N, kChkSlices) = op;
+                            SHG_AT(sl, (size_t)N * N + base + k, (size_t)2 * N * N, kChkSlices) = os;
                         }
                     }
                     if (s == K) {
@@ -146,6 +149,7 @@ __global__ void __launch_bounds__(ResShape<N, CS_, MINB_, G_>::THREADS, MINB_)
 #pragma unroll
                         for (int r = 0; r < E; ++r) {
                             const int k = spec_index<N, G>(t, r);
+                            march_leave(vp[r], vs[r], cprev, d);
                             SHG_AT(d.Pout, base + k, (size_t)N * N, kChkResidentLoad) = vp[r];
                             SHG_AT(d.Sout, base + k, (size_t)N * N, kChkResidentLoad) = vs[r];
                             aS += (double)vs[r].x * vs[r].x + (double)vs[r].y * vs[r].y;
@@ -154,9 +158,11 @@ __global__ void __launch_bounds__(ResShape<N, CS_, MINB_, G_>::THREADS, MINB_)
                         block_add_double_res(aS, d.acc + 1);
                         block_add_double_res(aP, d.acc + 2);
                     } else {
-                        const float4 c2 = ccur;
 #pragma unroll
-                        for (int r = 0; r < E; ++r) rk4_point(vp[r], vs[r], c2, d);
+                        for (int r = 0; r < E; ++r) {
+                            march_turn(vs[r], ccur);
+                            rk4_march(vp[r], vs[r], d);
+                        }
                         fft_spec_to_nat<N, G, +1, false, 1, G + 1, true>(vp, t, rsc, tab);
                         fft_spec_to_nat<N, G, +1, false, 1, G + 1, true>(vs, t, rsc, tab);
 #pragma unroll

@@ -389,7 +389,7 @@ int ThermalSolve::cwes(float power, float waist, float focal) {
     }
     h_desc_.slices = slices_;
     TH_CUDA(cudaMemcpyAsync(d_desc_, &h_desc_, sizeof(InstDesc), cudaMemcpyHostToDevice, st_));
-    TH_CUDA(launch_setup(d_desc_, 1, (int)nn, nz_, st_));
+    TH_CUDA(launch_setup(d_desc_, 1, (int)nn, nz_, false, st_));
     if (slices_) {
         TH_CUDA(cudaMemcpyAsync(slices_, h_desc_.P, nn * sizeof(float2), cudaMemcpyDeviceToDevice, st_));
         TH_CUDA(cudaMemcpyAsync(slices_ + nn, h_desc_.S, nn * sizeof(float2), cudaMemcpyDeviceToDevice, st_));
