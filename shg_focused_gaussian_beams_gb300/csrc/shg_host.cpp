@@ -96,8 +96,9 @@ float crystal_index(int crystal, float L, float T) {
 }
 
 // Scales of the marched fields (shg_march.cuh): they make both coupling constants of dA/dz equal
-// to 1. Without coupling (d_eff = 0, or so small that its square underflows) the fields are held
-// so small that the products vanish against them and p^2 underflows to zero.
+// to 1. Without coupling (d_eff = 0, or below 1e-12 pm/V, where kp < 2^-60 and p^2 would
+// underflow) the fields are held so small that the products vanish against them and p^2 is zero:
+// the fields diffract and are absorbed, and an SH that starts at zero stays zero.
 static void march_scales(InstDesc &d) {
     const bool coupled = std::fabs(d.kp) >= 0x1p-60f && std::fabs(d.ks) >= 0x1p-60f;
     d.ss = coupled ? d.kp : 0x1p-60f;
