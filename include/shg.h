@@ -202,7 +202,7 @@ int shg_batch_launch_count(shg_batch *b, int *launches);
  * Resident variants also differ in the line-FFT split (n = 64: 8 x 8 or 16 x 4 points).
  * Unless the environment variable SHG_MARCH is "streaming", "resident" (default variants)
  * or lists a schedule per grid ("64:1/1,128:4/2,256:16/2", "64:1/1/4", "64:streaming",
- * "128:coop"), the first run times every candidate on the class's own solves and keeps the
+ * "128:coop", "256:group"), the first run times every candidate on the class's own solves and keeps the
  * fastest (cached per device and class shape for the process). A batch of one solve has one
  * more candidate, "coop": the whole march in one cooperative launch (row and column passes
  * of the streaming kernels, bit-identical, separated by grid-wide barriers whose waits are
@@ -213,7 +213,8 @@ int shg_batch_autotune(shg_batch *b, void *stream);
  * persistent cooperative grid (a batch of one solve only; cluster_size and ctas_per_sm
  * unused), resident = 3 the cluster march (n in {64, 128, 256}: each solve in one cluster
  * of 8 / 16 / 16 CTAs of 512 threads, one thread per point in the pointwise phase;
- * cluster_size and ctas_per_sm unused), else the resident variant with cluster_size CTAs per cluster and ctas_per_sm
+ * cluster_size and ctas_per_sm unused), resident = 4 the persistent groups of blocks (n in
+ * {64, 128, 256}; cluster_size and ctas_per_sm unused), else the resident variant with cluster_size CTAs per cluster and ctas_per_sm
  * CTAs per SM (variants: n <= 32 (1, 1); n = 64 (1, 1), (1, 2), (2, 2), (2, 4); n = 128
  * (2, 1), (4, 1), (4, 2); n = 256 (8, 1), (16, 1), (16, 2)). SHG_ERR_UNSUPPORTED if the
  * variant does not exist or fit. */

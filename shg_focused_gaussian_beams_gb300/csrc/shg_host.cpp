@@ -210,7 +210,7 @@ int ensure_twiddles(int device) {
     for (const float2 *addr : {twiddle_symbol_address_march(), twiddle_symbol_address_thermal(),
                                twiddle_symbol_address_adjoint(), twiddle_symbol_address_resident(),
                                twiddle_symbol_address_resident128(), twiddle_symbol_address_resident256(),
-                               twiddle_symbol_address_cluster_pt()}) {
+                               twiddle_symbol_address_cluster_pt(), twiddle_symbol_address_group()}) {
         void *p = const_cast<float2 *>(addr);
         if (!p) {
             set_error("twiddle table symbol unavailable");
@@ -223,11 +223,12 @@ int ensure_twiddles(int device) {
 }
 
 // Name of a class schedule: "streaming", "coop" (persistent grid), "cluster" (one cluster
-// per solve, one thread per point) or "cs/minb/g".
+// per solve, one thread per point), "group" (persistent groups of blocks) or "cs/minb/g".
 std::string schedule_label(bool resident, const ResidentVariant &v) {
     if (!resident) return "streaming";
     if (v.cs == 0) return "coop";
     if (v.cs == -1) return "cluster";
+    if (v.cs == -2) return "group";
     return std::to_string(v.cs) + "/" + std::to_string(v.minb) + "/" + std::to_string(v.g);
 }
 
@@ -332,7 +333,7 @@ class Batch {
         }
         // schedule per class from SHG_MARCH: "auto" (default: the autotuner picks at the first
         // run), "streaming", "resident" (default variants), or a list "n:streaming" /
-        // "n:cs/minb" / "n:coop" / "n:cluster" per grid (e.g. "64:1/1,128:4/2,256:16/2";
+        // "n:cs/minb" / "n:coop" / "n:cluster" / "n:group" per grid (e.g. "64:1/1,128:4/2,256:16/2";
         // unlisted grids: autotuner; "coop", the persistent cooperative grid, applies to a
         // batch of one solve; "cluster" runs each solve in one cluster of the cluster march)
         const char *mode = std::getenv("SHG_MARCH");
@@ -359,6 +360,15 @@ class Batch {
                         c.resident = true;
                         c.var = ResidentVariant{0, 0, 0};
                         c.tuned = true;
+                    }
+                } else if (v == "group") {
+                    int mg = 0;
+                    if (prepare_resident(c.n, ResidentVariant{-2, 0, 0}, &mg) == cudaSuccess && mg > 0) {
+                        c.resident = true;
+                        c.var = ResidentVariant{-2, 0, 0};
+                        c.tuned = true;
+                    } else {
+                        cudaGetLastError();
                     }
                 } else if (v == "cluster") {
                     if (cluster_pt_size(c.n) > 0) {
@@ -389,7 +399,7 @@ class Batch {
             side_events_.push_back(e2);
         }
         if (!fork_event_) SHG_CUDA(cudaEventCreateWithFlags(&fork_event_, cudaEventDisableTiming));
-        SHG_CUDA(cudaMalloc(&d_counters_, 64 * sizeof(int)));
+        SHG_CUDA(cudaMalloc(&d_counters_, kCounterBytes));
         SHG_CUDA(cudaMalloc(&d_lists_, lists.size() * sizeof(int)));
         SHG_CUDA(cudaMemcpy(d_lists_, lists.data(), lists.size() * sizeof(int), cudaMemcpyHostToDevice));
         SHG_CUDA(cudaMemset(pool_, 0, pool_bytes_));
@@ -560,6 +570,13 @@ class Batch {
                 else
                     cudaGetLastError();
             }
+            if (c.count > 1) {  // persistent groups of blocks
+                int mc = 0;
+                if (prepare_resident(c.n, ResidentVariant{-2, 0, 0}, &mc) == cudaSuccess && mc > 0)
+                    cands.push_back({true, ResidentVariant{-2, 0, 0}, mc});
+                else
+                    cudaGetLastError();
+            }
             float best = 1e30f;
             int bi = 0;
             c.trials.clear();
@@ -572,7 +589,7 @@ class Batch {
                     rc = enqueue_inputs(st);
                     if (rc) break;
                     if (launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, true, st) != cudaSuccess ||
-                        cudaMemsetAsync(d_counters_, 0, 64 * sizeof(int), st) != cudaSuccess ||
+                        cudaMemsetAsync(d_counters_, 0, kCounterBytes, st) != cudaSuccess ||
                         cudaEventRecord(a, st) != cudaSuccess) {
                         rc = SHG_ERR_CUDA;
                         break;
@@ -735,6 +752,16 @@ class Batch {
                 c.resident = true;
                 c.var = ResidentVariant{-1, 1, 0};
                 c.max_clusters = mc;
+            } else if (resident == 4) {
+                int mc = 0;
+                if (prepare_resident(n, ResidentVariant{-2, 0, 0}, &mc) != cudaSuccess || mc < 1) {
+                    cudaGetLastError();
+                    set_error("set_schedule: the persistent groups run grids 64, 128 and 256 where a group fits");
+                    return SHG_ERR_UNSUPPORTED;
+                }
+                c.resident = true;
+                c.var = ResidentVariant{-2, 0, 0};
+                c.max_clusters = mc;
             } else {
                 ResidentVariant vs[16];
                 const int nv = resident_variants(n, vs, 16);
@@ -770,7 +797,7 @@ class Batch {
         }
         SHG_TRY_INT(enqueue_inputs(st));
         SHG_CUDA(launch_setup(d_desc_, (int)desc_.size(), max_nn_, max_nz_, true, st));
-        SHG_CUDA(cudaMemsetAsync(d_counters_, 0, 64 * sizeof(int), st));
+        SHG_CUDA(cudaMemsetAsync(d_counters_, 0, kCounterBytes, st));
         const int nc = (int)classes_.size();
         std::vector<cudaEvent_t> ev(2 * nc + 1);
         for (auto &e : ev) SHG_CUDA(cudaEventCreate(&e));
@@ -803,6 +830,7 @@ class Batch {
                    : !c.resident                   ? std::string("streaming")
                    : c.var.cs == 0                 ? std::string("coop (persistent grid)")
                    : c.var.cs == -1                ? std::string("cluster march")
+                   : c.var.cs == -2                ? std::string("persistent groups")
                                                    : "resident cs=" + std::to_string(c.var.cs) + " minb=" +
                                                        std::to_string(c.var.minb) + " g=" + std::to_string(c.var.g);
             if (!c.trials.empty()) {
@@ -983,7 +1011,7 @@ class Batch {
                 SHG_CUDA(cudaMemcpyAsync(desc_[i].slices + nn, desc_[i].S, nn * sizeof(float2),
                                          cudaMemcpyDeviceToDevice, st));
             }
-        SHG_CUDA(cudaMemsetAsync(d_counters_, 0, 64 * sizeof(int), st));
+        SHG_CUDA(cudaMemsetAsync(d_counters_, 0, kCounterBytes, st));
         // classes in descending grid size; concurrently on side streams unless timed
         std::vector<int> order(classes_.size());
         for (int i = 0; i < (int)order.size(); ++i) order[i] = i;
@@ -1012,6 +1040,14 @@ class Batch {
             unsigned *bar = reinterpret_cast<unsigned *>(d_counters_ + 40 + 2 * ci);
             if (rec) SHG_TRY_INT(rec->begin("coop<" + std::to_string(k.n) + ">", 32.0 * k.pt_steps, st));
             SHG_CUDA(launch_coop(k.n, d_desc_, list, bar, d_counters_ + 63, st));
+            if (rec) SHG_TRY_INT(rec->end(st));
+            return SHG_OK;
+        }
+        if (k.resident && k.var.cs == -2) {
+            // the persistent groups: words of grid 64, 128, 256 after the first 64, error word 63
+            unsigned *words = reinterpret_cast<unsigned *>(d_counters_ + 64) + (k.n == 64 ? 0 : k.n == 128 ? 1 : 2) * kGroupWords;
+            if (rec) SHG_TRY_INT(rec->begin("group<" + std::to_string(k.n) + ">", 32.0 * k.pt_steps, st));
+            SHG_CUDA(launch_group(k.n, d_desc_, list, k.count, words, d_counters_ + 63, st));
             if (rec) SHG_TRY_INT(rec->end(st));
             return SHG_OK;
         }
@@ -1093,6 +1129,8 @@ class Batch {
     bool desc_dirty_ = true;
     cudaGraphExec_t graph_exec_ = nullptr;
     cudaStream_t capture_stream_ = nullptr;
+    // job counters, barrier and error words of a run: 64 words, then those of the persistent groups
+    static constexpr size_t kCounterBytes = (64 + 3 * (size_t)kGroupWords) * sizeof(int);
     int *d_counters_ = nullptr;
     std::vector<std::pair<std::string, float>> mix_;  // concurrent-run trials of the autotuner
     std::vector<cudaStream_t> side_streams_;
@@ -1882,7 +1920,7 @@ int shg_check_status(int *enabled, int *site, long long *value) {
     unsigned long long first = 0;
     for (auto take : {check_word_take_march, check_word_take_resident64, check_word_take_resident128,
                       check_word_take_resident256, check_word_take_cluster_pt, check_word_take_thermal,
-                      check_word_take_heat_tma, check_word_take_heat_block, check_word_take_adjoint}) {
+                      check_word_take_heat_tma, check_word_take_heat_block, check_word_take_group, check_word_take_adjoint}) {
         const unsigned long long w = take();
         if (w == ~0ull) {
             set_error("shg_check_status: status word unreadable");

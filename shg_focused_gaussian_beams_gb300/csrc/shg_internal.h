@@ -30,6 +30,7 @@ const float2 *twiddle_symbol_address_resident();
 const float2 *twiddle_symbol_address_resident128();
 const float2 *twiddle_symbol_address_resident256();
 const float2 *twiddle_symbol_address_cluster_pt();
+const float2 *twiddle_symbol_address_group();
 
 // Check build (shg_check.cuh): each kernel translation unit's first failed check, read and
 // cleared (0: none; ~0: unreadable); always 0 in other builds.
@@ -41,6 +42,7 @@ unsigned long long check_word_take_cluster_pt();
 unsigned long long check_word_take_thermal();
 unsigned long long check_word_take_heat_tma();
 unsigned long long check_word_take_heat_block();
+unsigned long long check_word_take_group();
 unsigned long long check_word_take_adjoint();
 cudaError_t launch_check_selftest(long long value);
 
@@ -49,7 +51,8 @@ struct ResidentVariant {
     int cs, minb, g;  // cluster size, CTAs per SM, threads per line (FFT split N = (N/g) x g);
                       // cs == 0: the persistent cooperative grid of one solve (launch_coop);
                       // cs == -1: one cluster per solve, one thread per point in the
-                      // pointwise phase (launch_cluster_pt)
+                      // pointwise phase (launch_cluster_pt); cs == -2: persistent groups of
+                      // blocks (launch_group)
 };
 int resident_variants(int n, ResidentVariant *out, int max_out);
 ResidentVariant resident_default(int n);
@@ -76,6 +79,13 @@ bool line_length_supported(int n);
 int cluster_pt_size(int n);
 cudaError_t prepare_cluster_pt(int n, int *max_clusters);
 cudaError_t launch_cluster_pt(int n, const InstDesc *inst, const int *list, int count, cudaStream_t st);
+// shg_group.cu: the march of `njobs` solves (list[0..njobs)) by persistent groups of blocks with
+// bounded barriers, one cooperative launch (n in {64, 128, 256}). words: kGroupWords zeroed words;
+// err: zeroed, set when a barrier wait gave up. inst == nullptr only counts the groups that fit
+// co-resident (max_groups).
+constexpr int kMaxGroups = 512, kGroupWords = 1 + 2 * kMaxGroups;
+cudaError_t launch_group(int n, const InstDesc *inst, const int *list, int njobs, unsigned *words, int *err,
+                         cudaStream_t st, int *max_groups = nullptr);
 cudaError_t launch_dft2d(int n, int sign, const float2 *in, float2 *out, cudaStream_t st);
 cudaError_t launch_dft_rows(int n, int sign, const float2 *in, float2 *out, cudaStream_t st, int fields = 1);
 

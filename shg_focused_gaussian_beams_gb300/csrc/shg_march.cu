@@ -20,6 +20,7 @@
 #include "shg_internal.h"
 #include "shg_coop.cuh"
 #include "shg_march.cuh"
+#include "shg_stream.cuh"
 
 namespace shg {
 
@@ -76,20 +77,6 @@ __global__ void k_setup_steps(const InstDesc *__restrict__ inst, int n_inst, int
     }
 }
 
-__device__ __forceinline__ void block_add_double(double v, double *dst) {
-    __shared__ double red[32];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = (l < (int)(blockDim.x >> 5)) ? red[l] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (l == 0 && v != 0.0) atomicAdd(dst, v);
-    }
-}
-
 // Efields.h:74-104 (pump) and Efields.h:107-126 + 32-71 (propagators), with the float
 // operations of the reference kept in order (no contraction); only cosf/sinf/expf are the
 // device's. Grid: (chunks of 4*blockDim pixels, solves).
@@ -135,98 +122,18 @@ __global__ void k_setup_fields(const InstDesc *__restrict__ inst) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Row pass. Block = 256 threads = 256/G lines of one solve; mode from the stage s:
-//   s == 0           : RK4(z_0), backward transform along x, store in frequency order;
-//   0 < s < nsteps   : forward transform along x, RK4(z_{s-1}), RK4(z_s), backward;
-//   s == nsteps      : forward transform along x, RK4(z_{s-1}), capture, power sums.
+// Row pass (RowShape, rows_body: shg_stream.cuh).
+// (two blocks per SM from N = 128 on: at the 142 registers the compiler takes freely for N = 256 only
+// one fits)
 template <int N>
-struct RowShape {
-    static constexpr int G = LineShape<N>::G;
-    static constexpr int TPB = (N * G < 256) ? N * G : 256;  // threads per block
-    static constexpr int LPB = TPB / G;                      // lines per block
-    static constexpr int BPI = N / LPB;                      // blocks per solve
-};
-
-template <int N>
-__global__ void __launch_bounds__(RowShape<N>::TPB) k_rows(const InstDesc *__restrict__ inst, const int *__restrict__ list, int s) {
-    constexpr int G = LineShape<N>::G, E = N / G, LPB = RowShape<N>::LPB, BPI = RowShape<N>::BPI;
+__global__ void __launch_bounds__(RowShape<N>::TPB, N >= 128 ? 2 : 0) k_rows(const InstDesc *__restrict__ inst, const int *__restrict__ list, int s) {
+    constexpr int G = LineShape<N>::G, LPB = RowShape<N>::LPB, BPI = RowShape<N>::BPI;
     constexpr int SC = LineScratch<N, G>::SIZE;
-    static_assert(N % LPB == 0, "blocks must not straddle solves");
     __shared__ float2 scratch[LPB * SC];
     const InstDesc &d = inst[list[blockIdx.x / BPI]];
     if (!check_solve<N>(d, s)) return;  // whole block (d and s are block-uniform)
-    constexpr size_t NN = (size_t)N * N;
-    const float2 *__restrict__ tab = g_twiddle + N;
-    const int line = (blockIdx.x % BPI) * LPB + threadIdx.x / G;
-    const int t = threadIdx.x % G;
-    float2 *sc = scratch + (threadIdx.x / G) * SC;
-    const size_t base = (size_t)line * N;
-    float2 vp[E], vs[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-        vp[j] = SHG_AT(d.P, base + t + G * j, NN, kChkRowsGlobal);
-        vs[j] = SHG_AT(d.S, base + t + G * j, NN, kChkRowsGlobal);
-    }
-    if (s == 0) {
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-            march_enter(vp[j], vs[j], d);
-            rk4_march(vp[j], vs[j], d);
-        }
-        fft_nat_to_spec<N, G, +1>(vp, t, sc, tab);
-        fft_nat_to_spec<N, G, +1>(vs, t, sc, tab);
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-            const int k = spec_index<N, G>(t, r);
-            SHG_AT(d.P, base + k, NN, kChkRowsGlobal) = vp[r];
-            SHG_AT(d.S, base + k, NN, kChkRowsGlobal) = vs[r];
-        }
-        return;
-    }
-    fft_nat_to_spec<N, G, -1>(vp, t, sc, tab);
-    fft_nat_to_spec<N, G, -1>(vs, t, sc, tab);
-    const float4 c1 = d.stepc[s - 1];
-#pragma unroll
-    for (int r = 0; r < E; ++r) rk4_march(vp[r], vs[r], d);
-    if (d.slices && s < d.nz) {
-        float2 *sl = d.slices + (size_t)s * 2 * N * N;
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-            const int k = spec_index<N, G>(t, r);
-            float2 op = vp[r], os = vs[r];
-            march_leave(op, os, c1, d);
-            SHG_AT(sl, base + k, 2 * NN, kChkSlices) = op;
-            SHG_AT(sl, NN + base + k, 2 * NN, kChkSlices) = os;
-        }
-    }
-    if (s == d.nsteps) {
-        double aS = 0.0, aP = 0.0;
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-            const int k = spec_index<N, G>(t, r);
-            march_leave(vp[r], vs[r], c1, d);
-            SHG_AT(d.Pout, base + k, NN, kChkRowsGlobal) = vp[r];
-            SHG_AT(d.Sout, base + k, NN, kChkRowsGlobal) = vs[r];
-            aS += (double)vs[r].x * vs[r].x + (double)vs[r].y * vs[r].y;
-            aP += (double)vp[r].x * vp[r].x + (double)vp[r].y * vp[r].y;
-        }
-        block_add_double(aS, d.acc + 1);
-        block_add_double(aP, d.acc + 2);
-        return;
-    }
-    const float4 c2 = d.stepc[s];
-#pragma unroll
-    for (int r = 0; r < E; ++r) {
-        march_turn(vs[r], c2);
-        rk4_march(vp[r], vs[r], d);
-    }
-    fft_spec_to_nat<N, G, +1>(vp, t, sc, tab);
-    fft_spec_to_nat<N, G, +1>(vs, t, sc, tab);
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-        SHG_AT(d.P, base + t + G * j, NN, kChkRowsGlobal) = vp[j];
-        SHG_AT(d.S, base + t + G * j, NN, kChkRowsGlobal) = vs[j];
-    }
+    rows_body<N>(d, (blockIdx.x % BPI) * LPB + threadIdx.x / G, threadIdx.x % G, s, scratch + (threadIdx.x / G) * SC,
+                 g_twiddle + N);
 }
 
 // Row pass for one to three solves: the same work as k_rows with one thread per point.
@@ -337,30 +244,6 @@ __global__ void __launch_bounds__(PtRowShape<N>::TPB) k_rows_pt(const InstDesc *
     rows_pt_body<N>(d, (blockIdx.x % Sh::BPI) * Sh::LPB, s, scratch, lines[0], lines[1], g_twiddle + N);
 }
 
-// The column pass of k_cols for column x of field f (0 pump, 1 SH) of solve d, lane t of the
-// column's G lanes; the TC columns of a group transpose through sc (interleaved, stride TC)
-// and synchronise the block (BS) or, when the group is one warp, the warp.
-template <int N, int TC, bool BS>
-__device__ __forceinline__ void cols_body(const InstDesc &d, int x, int f, int t, float2 *sc) {
-    constexpr int G = LineShape<N>::G, E = N / G;
-    const float2 *__restrict__ tab = g_twiddle + N;
-    float2 *F = f == 0 ? d.P : d.S;
-    const float2 *__restrict__ H = f == 0 ? d.Hp : d.Hs;
-    constexpr size_t NN = (size_t)N * N;
-    // propagator values first: their latency overlaps the transform
-    float2 h[E];
-    hprop_load<N>(H, x, t, h);
-    float2 v[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) v[j] = SHG_AT(F, (size_t)(t + G * j) * N + x, NN, kChkColsGlobal);
-    fft_nat_to_spec<N, G, +1, BS, TC, G>(v, t, sc, tab);
-#pragma unroll
-    for (int r = 0; r < E; ++r) v[r] = c_mul(v[r], h[r]);
-    fft_spec_to_nat<N, G, -1, BS, TC, G>(v, t, sc, tab);
-#pragma unroll
-    for (int j = 0; j < E; ++j) SHG_AT(F, (size_t)(t + G * j) * N + x, NN, kChkColsGlobal) = v[j];
-}
-
 // Column pass. Block = TC columns x G threads (lane = column + TC * t) so that every
 // load and store is a run of TC consecutive complex values; blockIdx.y = field (pump, SH).
 template <int N, int TC>
@@ -370,7 +253,7 @@ __global__ void __launch_bounds__(TC * LineShape<N>::G) k_cols(const InstDesc *_
     const int c = threadIdx.x % TC;
     const InstDesc &d = inst[list[blockIdx.x / BPI]];
     if (!SHG_REQUIRE(d.n == N, kChkDescriptor, d.n)) return;
-    cols_body<N, TC, true>(d, (blockIdx.x % BPI) * TC + c, blockIdx.y, threadIdx.x / TC, scratch + c);
+    cols_body<N, TC, true>(d, (blockIdx.x % BPI) * TC + c, blockIdx.y, threadIdx.x / TC, scratch + c, g_twiddle + N);
 }
 
 // ---------------------------------------------------------------------------------------

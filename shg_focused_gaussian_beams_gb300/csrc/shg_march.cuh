@@ -68,8 +68,9 @@ __device__ __forceinline__ void dadz_point(float2 P, float2 S, float4 c, float h
 // this frame the coupling constants of dA/dz are 1,
 //   dp = i s conj(p) - hp p,   ds = i p^2 - (tpa0 + tpa1s |s|^2) s,
 // so an evaluation takes 15 multiply-adds instead of 22 (eight per point and z step, of 475
-// instructions in all: 24 solves of 64x64x200 1.54 -> 1.38 ms, one of 256x256x400 3.04 -> 2.85 ms). The frame is the same for all
-// stages of a slice; going to the next slice turns s by the constant angle d = (z_s - z_{s-1}) dk.
+// instructions in all: 24 solves of 64x64x200 1.54 -> 1.38 ms, one of 256x256x400 3.04 -> 2.85 ms).
+// The frame is the same for all stages of a slice; going to the next slice turns s by the
+// constant angle d = (z_s - z_{s-1}) dk.
 __device__ __forceinline__ void dads_point(float2 p, float2 s, float hp, float tpa0, float tpa1s, float2 &dp, float2 &ds) {
     const float mx = hp * p.x, my = hp * p.y;
     dp.x = fmaf(s.x, p.y, fmaf(-s.y, p.x, -mx));

@@ -73,6 +73,10 @@ cudaError_t prepare_resident(int n, ResidentVariant v, int *max_clusters) {
         return e;
     }
     if (v.cs == -1) return prepare_cluster_pt(n, max_clusters);
+    if (v.cs == -2) {
+        *max_clusters = 0;
+        return launch_group(n, nullptr, nullptr, 0, nullptr, nullptr, nullptr, max_clusters);
+    }
     switch (n) {
         case 16: case 32: case 64: return prepare_resident_small(n, v.cs, v.minb, v.g, max_clusters);
         case 128: return prepare_resident_128(v.cs, v.minb, v.g, max_clusters);

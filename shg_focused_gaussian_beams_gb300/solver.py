@@ -321,10 +321,11 @@ class Sweep:
     def set_schedule(self, n, resident=True, cluster_size=1, ctas_per_sm=1, threads_per_line=None):
         """Fix the schedule of the grid-n class: streaming (resident=False), a resident variant
         (optionally with its line-FFT split), resident="coop", the persistent cooperative
-        grid of a batch of one solve, or resident="cluster", one thread-block cluster per solve
-        with one thread per point in the pointwise phase."""
-        if resident in ("coop", "cluster"):
-            mode = 2 if resident == "coop" else 3
+        grid of a batch of one solve, resident="cluster", one thread-block cluster per solve
+        with one thread per point in the pointwise phase, or resident="group", persistent groups
+        of blocks."""
+        if resident in ("coop", "cluster", "group"):
+            mode = {"coop": 2, "cluster": 3, "group": 4}[resident]
             check(lib().shg_batch_set_schedule(self._b, int(n), mode, 0, 0), "shg_batch_set_schedule")
             return
         if resident and threads_per_line:
