@@ -260,6 +260,10 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
     k_heat_block(float *__restrict__ Tf, const float *__restrict__ Ti, const float *__restrict__ QK,
                  const __grid_constant__ HeatCoef c, const __grid_constant__ HeatBlockGrid g) {
     static_assert(K <= kMaxLevels && K <= kRing - kAhead, "the Q/k ring holds the planes of K levels");
+    // Short chunks: the next sweep's blocks may start as soon as all of these have, so that their
+    // set-up up to their own wait overlaps this launch's last planes. Of long ones it takes SM
+    // slots for nothing (256x256x400 oven 48.4 us per sweep with it, 47.8 without).
+    if (g.zc <= 16) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int R = kRows, PL = plane_floats(THREADS, R);
     extern __shared__ __align__(16) float hb_smem[];
     const int vx = g.vx, rows = R * (THREADS / vx), row = 4 * vx;
@@ -475,24 +479,46 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
         leave(s);
     };
 
+    // A step whose levels have nothing to compute yet: plane p only moves into place.
+    auto skip = [&](int s) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) cc[0][k] = cur[k];
+        leave(s);
+    };
+    // The first step is one, and so is the second unless the chunk starts at the first slice: up to
+    // half of the steps of the two- and four-plane chunks that small grids are cut into.
     int p = plo, s = 0;
-    for (;;) {  // slots as constants: four steps to an iteration
-        s = 0;
-        if (arrive(0)) break;
-        body(0, p);
-        if (++p > pend) return;
+    bool in_range = !arrive(0);
+    if (in_range) {
+        skip(0);
+        ++p;
         s = 1;
-        if (arrive(1)) break;
-        body(1, p);
+        in_range = !arrive(1);
+    }
+    if (in_range) {
+        if (plo > 0)
+            skip(1);
+        else
+            body(1, p);
         if (++p > pend) return;
-        s = 2;
-        if (arrive(2)) break;
-        body(2, p);
-        if (++p > pend) return;
-        s = 3;
-        if (arrive(3)) break;
-        body(3, p);
-        if (++p > pend) return;
+        for (;;) {  // slots as constants: four steps to an iteration
+            s = 2;
+            if (arrive(2)) break;
+            body(2, p);
+            if (++p > pend) return;
+            s = 3;
+            if (arrive(3)) break;
+            body(3, p);
+            if (++p > pend) return;
+            s = 0;
+            if (arrive(0)) break;
+            body(0, p);
+            if (++p > pend) return;
+            s = 1;
+            if (arrive(1)) break;
+            body(1, p);
+            if (++p > pend) return;
+        }
     }
     for (;;) {
         body_any(s, p);
@@ -524,18 +550,22 @@ bool heat_block_supported(int nx, int ny, int nz) {
 }
 
 // Tiling and sweeps per launch for a grid: the candidate whose modelled time per sweep is
-// least. The model's constants (cycles at 1.92 GHz) were fitted to the measured sweeps below:
-// a launch and its prologue, and per z step the chain through the levels plus the issue of the
-// warps that share a scheduler; a sweep that does not fit L2 cannot beat 2600 bytes per cycle.
-// Two sweeps per launch halve the memory traffic and the launches but add two rows of halo on
-// each side and two planes at each chunk's ends; three and four were built too and lost (their
-// state spills at the 128 registers of two 256-thread blocks per SM). us per sweep on GB300,
-// the TMA-staged sweep (shg_heat_tma.cu) -> one / two sweeps per launch here:
-//   32x32x50    open top 16.6 -> 4.6 / 5.1,    oven 10.4 -> 2.9 / 2.7
-//   64x64x200   open top 16.6 -> 6.4 / 6.9,    oven 10.5 -> 4.5 / 3.8
-//   100x100x75  open top 16.6 -> 6.1 / 6.8,    oven 12.4 -> 4.8 / 4.1
-//   128x128x200 open top 20.7 -> 10.8 / 10.7,  oven 14.6 -> 8.3 / 7.6
-//   256x256x400 open top 81.0 -> 71.5 / 65.5,  oven 69.9 -> 63.8 / 46.5
+// least. The model (cycles at 1.92 GHz, fitted to the sweeps measured below): 4300 cycles per wave
+// of blocks (launch, set-up, first planes), then per z step that computes 1500 (2500 with two
+// sweeps in flight) at 16 warps per SM, a third of which is latency; with the open top's lateral
+// faces 1700 + 70000 / NX (their lanes' share of a warp falls with NX), 1.65 times that with two
+// sweeps. A launch that leaves slots free is marked up by a third: the next launch's early blocks
+// crowd onto the same SMs. A sweep that does not fit L2 cannot beat 2600 bytes per cycle. Two
+// sweeps per launch halve the memory traffic and the launches but add two rows of halo on each
+// side and two planes at each chunk's ends; three and four were built too and lost (their state
+// spills at the 128 registers of two 256-thread blocks per SM). us per sweep on GB300, the
+// TMA-staged sweep (shg_heat_tma.cu) -> one / two sweeps per launch here:
+//   32x32x50    open top 14.8 -> 4.4 / 4.8,   oven 10.6 -> 2.6 / 2.6
+//   64x64x200   open top 14.7 -> 5.6 / 6.4,   oven 10.6 -> 4.2 / 4.2
+//   100x100x75  open top 16.8 -> 4.7 / 5.8,   oven 11.6 -> 4.1 / 4.0
+//   128x128x200 open top 21.0 -> 9.6 / 9.8,   oven 14.8 -> 7.6 / 6.7
+//   200x200x150 open top 32.5 -> 19.5 / 19.4, oven 25.4 -> 16.6 / 14.2
+//   256x256x400 open top 86.2 -> 69.2 / 65.9, oven 71.4 -> 64.8 / 48.4
 // (47 us is the HBM copy rate for one sweep's 12 bytes per voxel.) At 256x256x400 with two
 // sweeps per launch: 79 warp instructions per four voxels and level of a warp, 51 % issue, FMA
 // pipe 23 % (the packed forms take it for two cycles), shared-memory latency the top stall.
@@ -543,8 +573,8 @@ static cudaError_t search_plan(int dev, int nx, int ny, int nz, int bc, int leve
     int sms = 0;
     cudaError_t e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    constexpr double kLaunch = 4200, kWave = 400, kBytesPerCycle = 2600, kL2 = 100e6;
-    const double chain = bc == 0 ? 500 : 100, issue = bc == 0 ? 340 : 312, bytes = 12.0 * nx * ny * nz;
+    constexpr double kWave = 4300, kBytesPerCycle = 2600, kL2 = 100e6;
+    const double bytes = 12.0 * nx * ny * nz;
     const int vecs = nx / 4;
     double best = 1e300;
     for (int K = levels ? levels : 1; K <= (levels ? levels : kMaxLevels); ++K)
@@ -557,13 +587,15 @@ static cudaError_t search_plan(int dev, int nx, int ny, int nz, int bc, int leve
                 if ((!whole_x && vx < 8) || (!whole_y && rows <= 2 * K)) continue;
                 const int ti = whole_x ? vecs : vx - 2, tx = (vecs + ti - 1) / ti;
                 const int tyi = whole_y ? ny : rows - 2 * K, ty = (ny + tyi - 1) / tyi;
-                const int bps = 512 / threads, warps = threads / 128;  // blocks per SM, warps per scheduler
+                const int bps = 512 / threads, warps = threads / 128;  // blocks per SM, warps per scheduler of one
                 const long long slots = (long long)bps * sms, tiles = (long long)tx * ty;
                 for (int nc = 1; nc <= nz; ++nc) {
                     const int zc = (nz + nc - 1) / nc;
                     const long long blocks = tiles * ((nz + zc - 1) / zc), waves = (blocks + slots - 1) / slots;
                     const double w = warps * (waves > 1 ? (double)bps : (double)((blocks + sms - 1) / sms));
-                    double cost = kLaunch + waves * (kWave + (zc + 2 * K) * K * (chain + issue * w));
+                    const double full = bc == 0 ? (1700 + 70000.0 / nx) * (K == 1 ? 1.0 : 1.65) : K == 1 ? 1500 : 2500;
+                    double cost = waves * (kWave + (zc + 2 * K - 2) * full * (0.35 + 0.65 * w / 4));
+                    if (waves == 1 && 5 * blocks < 4 * slots) cost *= 1.35;
                     if (bytes > kL2) cost = std::max(cost, bytes / kBytesPerCycle);
                     if (cost / K < best) {
                         best = cost / K;
