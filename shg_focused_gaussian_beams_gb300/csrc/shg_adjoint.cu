@@ -38,7 +38,9 @@ SHG_CHECK_TU(adjoint)
 // A and Fst hold the fields back to back (solve-major), acc[blockIdx.y] receives the sums.
 // TC columns per block: 16 when several solves fill the GPU, 4 for one to three solves
 // (N >= 64, so that a block holds whole warps).
-template <int N, int MODE, int TC>
+// CHAINED: launched by launch_dependent (the batched THERMAL pass; of the plain adjoint, whose replay
+// branch runs at another priority, programmatic launches cost 2 %).
+template <int N, int MODE, int TC, bool CHAINED>
 __global__ void __launch_bounds__(TC * LineShape<N>::G) k_colpass(float2 *A0, float2 *Fst0,
                                                              const InstDesc *__restrict__ dd, double *acc0) {
     constexpr int G = LineShape<N>::G, E = N / G;
@@ -63,6 +65,7 @@ __global__ void __launch_bounds__(TC * LineShape<N>::G) k_colpass(float2 *A0, fl
 #pragma unroll
         for (int r = 0; r < E; ++r) fv[r] = Fst[(size_t)spec_index<N, G>(t, r) * N + x];
     }
+    if constexpr (CHAINED) grid_dependency_wait();
     float2 v[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) v[j] = A[(size_t)(t + G * j) * N + x];
@@ -304,35 +307,36 @@ static int grid_for(int nn) {
 
 template <int N, int TC>
 static cudaError_t launch_colpass_tc(int mode, float2 *A, float2 *F, const InstDesc *d, double *acc, int solves,
-                                     cudaStream_t st) {
+                                     bool chained, cudaStream_t st) {
     constexpr int G = LineShape<N>::G;
     const dim3 grid(N / TC, 2 * solves);
+    if (chained)
+        return launch_dependent(mode == 0 ? k_colpass<N, 0, TC, true> : k_colpass<N, 2, TC, true>, grid, TC * G, st, A, F,
+                                d, acc);
     if (mode == 0)
-        k_colpass<N, 0, TC><<<grid, TC * G, 0, st>>>(A, F, d, acc);
-    else if (mode == 1)
-        k_colpass<N, 1, TC><<<grid, TC * G, 0, st>>>(A, F, d, acc);
+        k_colpass<N, 0, TC, false><<<grid, TC * G, 0, st>>>(A, F, d, acc);
     else
-        k_colpass<N, 2, TC><<<grid, TC * G, 0, st>>>(A, F, d, acc);
+        k_colpass<N, 1, TC, false><<<grid, TC * G, 0, st>>>(A, F, d, acc);
     return cudaGetLastError();
 }
 
 template <int N>
 static cudaError_t launch_colpass_t(int mode, float2 *A, float2 *F, const InstDesc *d, double *acc, int solves,
-                                    cudaStream_t st) {
+                                    bool chained, cudaStream_t st) {
     // narrow tiles only where a block still fills a warp (the sums use full-warp shuffles)
-    if (solves >= 4 || 4 * LineShape<N>::G < 32) return launch_colpass_tc<N, 16>(mode, A, F, d, acc, solves, st);
-    return launch_colpass_tc<N, 4>(mode, A, F, d, acc, solves, st);
+    if (solves >= 4 || 4 * LineShape<N>::G < 32) return launch_colpass_tc<N, 16>(mode, A, F, d, acc, solves, chained, st);
+    return launch_colpass_tc<N, 4>(mode, A, F, d, acc, solves, chained, st);
 }
 
 cudaError_t launch_colpass(int n, int mode, float2 *A, float2 *F, const InstDesc *d, double *acc, cudaStream_t st,
-                           int solves) {
-    if (solves < 1 || solves > 32767) return cudaErrorInvalidValue;
+                           int solves, bool chained) {
+    if (solves < 1 || solves > 32767 || mode == (chained ? 1 : 2)) return cudaErrorInvalidValue;
     switch (n) {
-        case 16: return launch_colpass_t<16>(mode, A, F, d, acc, solves, st);
-        case 32: return launch_colpass_t<32>(mode, A, F, d, acc, solves, st);
-        case 64: return launch_colpass_t<64>(mode, A, F, d, acc, solves, st);
-        case 128: return launch_colpass_t<128>(mode, A, F, d, acc, solves, st);
-        case 256: return launch_colpass_t<256>(mode, A, F, d, acc, solves, st);
+        case 16: return launch_colpass_t<16>(mode, A, F, d, acc, solves, chained, st);
+        case 32: return launch_colpass_t<32>(mode, A, F, d, acc, solves, chained, st);
+        case 64: return launch_colpass_t<64>(mode, A, F, d, acc, solves, chained, st);
+        case 128: return launch_colpass_t<128>(mode, A, F, d, acc, solves, chained, st);
+        case 256: return launch_colpass_t<256>(mode, A, F, d, acc, solves, chained, st);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -7,6 +7,25 @@
 
 namespace shg {
 
+// The passes of a z step form a chain, each reading what the one before it wrote. Launched with
+// programmatic serialisation, a pass starts while its predecessor drains, fetches what no pass
+// writes (propagator, coefficients) and waits here for the predecessor's results.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*k)(P...), dim3 grid, int threads, cudaStream_t st, A... a) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, P(a)...);
+}
+
 // Adds the block's k partial sums (k <= 6) to dst[0..k) with one FP64 atomic each.
 __device__ __forceinline__ void block_sum_doubles(double *v, int k, double *dst) {
     __shared__ double red[32][6];
@@ -129,7 +148,7 @@ __device__ __forceinline__ void rk4_vjp_point(float2 P, float2 S, float2 &cP, fl
 // RK4^T) work of the step boundary, and starts the next diffraction along x, so a z-step
 // costs one row and one column launch. The working state A / cotangent C holds the pump
 // then the SH field (n*n each); the column passes (k_colpass) see rows in natural
-// frequency order, as after launch_dft_rows(+1).
+// frequency order.
 template <int N>
 struct AdjRowShape {
     static constexpr int G = LineShape<N>::G;

@@ -19,6 +19,13 @@
 
 namespace shg {
 
+const float2 *twiddle_symbol_address_adjoint_th() {
+    void *p = nullptr;
+    cudaGetSymbolAddress(&p, g_twiddle);
+    return static_cast<const float2 *>(p);
+}
+SHG_CHECK_TU(adjoint_th)
+
 // coef[s*nn + i] = (kp, ks, tpa1, DKint_s) of pixel i for s < K; the running sum follows
 // the order of the thermal row pass (DKint_0 = DK_0, DKint_s = DKint_{s-1} + DK_s).
 __global__ void k_th_coef_table(const float *__restrict__ NP, const float *__restrict__ NS,
@@ -84,62 +91,226 @@ __device__ __forceinline__ void th_vjp_point(const float2 P, const float2 S, flo
     cs = c_add(cas, bs);
 }
 
-// Step boundary of the forward march in one pass over every solve's state X: RK4_th of step
-// sp (its second call, slice sp; skipped for sp < 0) with its input stored to save_w, then
-// the state stored to save_x, then RK4_th of step sn (its first call, slice sn; skipped for
-// sn < 0): the state crosses memory once per step boundary.
-__global__ void k_th_rk4_pair(float2 *X, float2 *save_w, float2 *save_x, const float4 *__restrict__ coef, int nn,
-                              int K, int sp, int sn, const InstDesc *__restrict__ dd) {
-    const int b = blockIdx.y;
+// Fused row passes. Between two column passes a step boundary finishes one diffraction along x,
+// applies the pointwise RK4_th (or its transpose) of the boundary and starts the next diffraction
+// along x, so a z step is one row and one column launch and the state crosses memory once per
+// launch. A block transforms LPB lines of the pump and of the SH at once, every thread E = N / G
+// points of one line in registers; between the transforms the lines lie in shared memory (in the
+// transforms' own scratch) and all threads take the points in turn, a point's coefficients and
+// stored states being fetched one point ahead. Instruction issue bounds the pass (69 % of the issue
+// slots at 16 x 256 x 256 points, 1.9 TB/s from HBM). Against separate transform and pointwise
+// passes, four launches per z step, each with the state through memory, us per z step forward /
+// gradient: 16 x 256 x 256 49/133 -> 34/103, 64 x 64 x 64 16/42 -> 12.6/32. The whole pass in
+// one cooperative launch with barriers among each solve's blocks was slower at every size (41/131
+// and 13.3/39.5; 7.3/19.9 against 5.4/11.2 for one 64 x 64 solve).
+//
+// SHAPE 0: 128 threads, which all transform; 1: the same lines with 256 threads; 2: half the lines
+// with 256 threads. 1 and 2 shorten the chain of points that a thread works through, for batches
+// that leave the SMs room (row_shape).
+template <int N, int SHAPE>
+struct ThRowShape {
+    static constexpr int G = LineShape<N>::G, E = N / G;
+    static constexpr int LMAX = (SHAPE == 2 ? 32 : 64) / G, LPB = LMAX < N ? LMAX : N;  // lines per field
+    static constexpr int FT = LPB * G;                                           // transform threads per field
+    static constexpr int TPB = SHAPE && LPB * N >= 256 ? 256 : 2 * FT;
+    static constexpr int BPI = N / LPB, PTS = LPB * N / TPB;                     // blocks per solve, points per thread
+    static constexpr int SC = LineScratch<N, G>::SIZE;
+    static constexpr int BLOCKS = 512 / TPB;  // resident blocks per SM (128 registers)
+    static_assert(FT % 32 == 0 && 2 * FT <= TPB && N % LPB == 0 && LPB * N % TPB == 0 && SC >= N, "row pass shape");
+};
+
+// Roles of a thread: transform role (line of field f, lane t) and point role (points i of the
+// block's LPB * N, consecutive threads consecutive points).
+template <int N, int SHAPE>
+struct ThRow {
+    using Sh = ThRowShape<N, SHAPE>;
+    static constexpr int G = Sh::G, E = Sh::E, LPB = Sh::LPB, SC = Sh::SC;
+    float2 *sm;
+    __device__ ThRow(float2 *s) : sm(s) {}
+    __device__ static bool transforms() { return threadIdx.x < 2 * Sh::FT; }
+    __device__ float2 *line() const { return sm + (threadIdx.x / G) * SC; }  // lines [0, LPB) pump, then SH
+    __device__ static size_t row() {  // this thread's row in the solve's state (pump, then SH)
+        const int fl = threadIdx.x / G, f = fl / LPB;
+        return ((size_t)f * N + blockIdx.x * LPB + fl % LPB) * N;
+    }
+    __device__ float2 &at(int f, int i) const { return sm[(f * LPB + i / N) * SC + i % N]; }
+    // rows of A (natural frequency order) -> lines in real space
+    __device__ void finish(const float2 *A, const float2 *tab) const {
+        if (!transforms()) return;
+        const int t = threadIdx.x % G;
+        const size_t r0 = row();
+        float2 v[E];
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = SHG_AT(A, r0 + t + G * j, (size_t)2 * N * N, kChkAdjoint);
+        fft_nat_to_spec<N, G, -1>(v, t, line(), tab);
+        __syncwarp();  // the line's lanes have read the scratch that it overwrites
+#pragma unroll
+        for (int r = 0; r < E; ++r) line()[spec_index<N, G>(t, r)] = v[r];
+    }
+    // lines in real space -> rows of A (natural frequency order)
+    __device__ void start(float2 *A, const float2 *tab) const {
+        if (!transforms()) return;
+        const int t = threadIdx.x % G;
+        const size_t r0 = row();
+        float2 v[E];
+#pragma unroll
+        for (int r = 0; r < E; ++r) v[r] = line()[spec_index<N, G>(t, r)];
+        fft_spec_to_nat<N, G, +1>(v, t, line(), tab);
+#pragma unroll
+        for (int j = 0; j < E; ++j) SHG_AT(A, r0 + t + G * j, (size_t)2 * N * N, kChkAdjoint) = v[j];
+    }
+};
+
+// Forward boundary of every solve: with sp >= 0 the end of the diffraction of step sp in A, whose
+// result W_sp goes to save_w, and RK4_th of step sp (its second call); otherwise the state at
+// (inP, inS), `stride` apart from solve to solve (inS null: no SH yet). The state X_{sp+1} goes to
+// save_x. With sn >= 0 RK4_th of step sn (its first call) and the start of its diffraction in A;
+// otherwise the state to out. Null pointers skip their stores, and the RK4 that nothing reads.
+template <int N, int SHAPE>
+__global__ void __launch_bounds__(ThRowShape<N, SHAPE>::TPB, ThRowShape<N, SHAPE>::BLOCKS)
+    k_th_rows_fwd(float2 *A0, const float2 *inP, const float2 *inS, size_t stride, float2 *save_w, float2 *save_x,
+                  float2 *out, const float4 *__restrict__ coef, int K, int sp, int sn,
+                  const InstDesc *__restrict__ dd) {
+    using Sh = ThRowShape<N, SHAPE>;
+    __shared__ float2 sm[2 * Sh::LPB * Sh::SC];
+    constexpr int NN = N * N, P = Sh::LPB * N;
+    const int b = blockIdx.y, base = blockIdx.x * P;  // this block's points of a field
     const InstDesc &d = dd[b];
-    float2 *P = X + (size_t)b * 2 * nn, *S = P + nn;
-    const size_t o = (size_t)b * 2 * nn;
-    const float4 *__restrict__ cp = coef + ((size_t)b * K + (sp < 0 ? 0 : sp)) * nn;
-    const float4 *__restrict__ cn = coef + ((size_t)b * K + (sn < 0 ? 0 : sn)) * nn;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-        float2 p = P[i], q = S[i];
+    const float2 *__restrict__ tab = g_twiddle + N;
+    const ThRow<N, SHAPE> rw(sm);
+    float2 *A = A0 + (size_t)b * 2 * NN;
+    const size_t o = (size_t)b * 2 * NN + base;
+    const float4 *__restrict__ cp = coef + ((size_t)b * K + (sp < 0 ? 0 : sp)) * NN + base;
+    const float4 *__restrict__ cn = coef + ((size_t)b * K + (sn < 0 ? 0 : sn)) * NN + base;
+    const bool second = sp >= 0 && (save_x || out || sn >= 0);
+    int i = threadIdx.x;
+    float4 vp = make_float4(0.f, 0.f, 0.f, 0.f), vn = vp;
+    if (second) vp = cp[i];
+    if (sn >= 0) vn = cn[i];
+    grid_dependency_wait();
+    if (sp >= 0) {
+        rw.finish(A, tab);
+        __syncthreads();
+    }
+    const float dz = d.dz;
+#pragma unroll 1
+    for (int j = 0; j < Sh::PTS; ++j, i += Sh::TPB) {
+        const float4 fp = vp, fn = vn;
+        if (j + 1 < Sh::PTS) {
+            if (second) vp = cp[i + Sh::TPB];
+            if (sn >= 0) vn = cn[i + Sh::TPB];
+        }
+        float2 p, q;
         if (sp >= 0) {
+            p = rw.at(0, i);
+            q = rw.at(1, i);
             if (save_w) {
                 save_w[o + i] = p;
-                save_w[o + nn + i] = q;
+                save_w[o + NN + i] = q;
             }
-            rk4_point_th(p, q, th_coef_of(cp[i], sp, d.dz), d);
+            if (second) rk4_point_th(p, q, th_coef_of(fp, sp, dz), d);
+        } else {
+            p = inP[b * stride + base + i];
+            q = inS ? inS[b * stride + base + i] : make_float2(0.f, 0.f);
         }
         if (save_x) {
             save_x[o + i] = p;
-            save_x[o + nn + i] = q;
+            save_x[o + NN + i] = q;
         }
-        if (sn >= 0) rk4_point_th(p, q, th_coef_of(cn[i], sn, d.dz), d);
-        P[i] = p;
-        S[i] = q;
+        if (sn >= 0) {
+            rk4_point_th(p, q, th_coef_of(fn, sn, dz), d);
+            rw.at(0, i) = p;  // each thread rewrites only the points it read
+            rw.at(1, i) = q;
+        } else if (out) {
+            out[o + i] = p;
+            out[o + NN + i] = q;
+        }
+    }
+    if (sn >= 0) {
+        __syncthreads();
+        rw.start(A, tab);
     }
 }
 
-// Step boundary of the reverse sweep in one pass over every solve's cotangent: RK4_th^T of
-// step sa at its first call's input Xa (skipped for sa < 0), then RK4_th^T of step sb at its
-// second call's input Wb (skipped for sb < 0).
-__global__ void k_th_vjp_pair(const float2 *__restrict__ Xa, const float2 *__restrict__ Wb, float2 *cot,
-                              const float4 *__restrict__ coef, int nn, int K, int sa, int sb,
-                              const InstDesc *__restrict__ dd) {
-    const int b = blockIdx.y;
+// Reverse boundary of every solve's cotangent C: with sa >= 0 the end of the adjoint diffraction
+// of step sa and RK4_th^T at its first call's input Xa, otherwise C as it is; with sb >= 0
+// RK4_th^T of step sb at its second call's input Wb and the start of its adjoint diffraction in C,
+// otherwise the cotangent to C.
+template <int N, int SHAPE>
+__global__ void __launch_bounds__(ThRowShape<N, SHAPE>::TPB, ThRowShape<N, SHAPE>::BLOCKS)
+    k_th_rows_bwd(float2 *C0, const float2 *__restrict__ Xa, const float2 *__restrict__ Wb,
+                  const float4 *__restrict__ coef, int K, int sa, int sb, const InstDesc *__restrict__ dd) {
+    using Sh = ThRowShape<N, SHAPE>;
+    __shared__ float2 sm[2 * Sh::LPB * Sh::SC];
+    constexpr int NN = N * N, P = Sh::LPB * N;
+    const int b = blockIdx.y, base = blockIdx.x * P;
     const InstDesc &d = dd[b];
-    const size_t o = (size_t)b * 2 * nn;
-    float2 *cP = cot + o, *cS = cP + nn;
-    const float4 *__restrict__ ca = coef + ((size_t)b * K + (sa < 0 ? 0 : sa)) * nn;
-    const float4 *__restrict__ cb = coef + ((size_t)b * K + (sb < 0 ? 0 : sb)) * nn;
-    const float hp = d.hp, t0 = d.tpa0, w6 = d.dz6;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-        float2 a = cP[i], c = cS[i];
-        if (sa >= 0) th_vjp_point(Xa[o + i], Xa[o + nn + i], a, c, th_coef_of(ca[i], sa, d.dz), hp, t0, w6);
-        if (sb >= 0) th_vjp_point(Wb[o + i], Wb[o + nn + i], a, c, th_coef_of(cb[i], sb, d.dz), hp, t0, w6);
-        cP[i] = a;
-        cS[i] = c;
+    const float2 *__restrict__ tab = g_twiddle + N;
+    const ThRow<N, SHAPE> rw(sm);
+    float2 *C = C0 + (size_t)b * 2 * NN;
+    const size_t o = (size_t)b * 2 * NN + base;
+    const float4 *__restrict__ ca = coef + ((size_t)b * K + (sa < 0 ? 0 : sa)) * NN + base;
+    const float4 *__restrict__ cb = coef + ((size_t)b * K + (sb < 0 ? 0 : sb)) * NN + base;
+    int i = threadIdx.x;
+    float4 va = make_float4(0.f, 0.f, 0.f, 0.f), vb = va;
+    float2 xp = make_float2(0.f, 0.f), xs = xp, wp = xp, ws = xp;
+    auto fetch_coef = [&](int k) {
+        if (sa >= 0) va = ca[k];
+        if (sb >= 0) vb = cb[k];
+    };
+    auto fetch_state = [&](int k) {
+        if (sa >= 0) {
+            xp = Xa[o + k];
+            xs = Xa[o + NN + k];
+        }
+        if (sb >= 0) {
+            wp = Wb[o + k];
+            ws = Wb[o + NN + k];
+        }
+    };
+    fetch_coef(i);
+    grid_dependency_wait();
+    fetch_state(i);
+    if (sa >= 0) {
+        rw.finish(C, tab);
+        __syncthreads();
+    }
+    const float dz = d.dz, hp = d.hp, t0 = d.tpa0, w6 = d.dz6;
+#pragma unroll 1
+    for (int j = 0; j < Sh::PTS; ++j, i += Sh::TPB) {
+        const float4 fa = va, fb = vb;
+        const float2 gp = xp, gs = xs, hw = wp, hs = ws;
+        if (j + 1 < Sh::PTS) {
+            fetch_coef(i + Sh::TPB);
+            fetch_state(i + Sh::TPB);
+        }
+        float2 p, q;
+        if (sa >= 0) {
+            p = rw.at(0, i);
+            q = rw.at(1, i);
+            th_vjp_point(gp, gs, p, q, th_coef_of(fa, sa, dz), hp, t0, w6);
+        } else {
+            p = C[base + i];
+            q = C[NN + base + i];
+        }
+        if (sb >= 0) {
+            th_vjp_point(hw, hs, p, q, th_coef_of(fb, sb, dz), hp, t0, w6);
+            rw.at(0, i) = p;  // each thread rewrites only the points it read
+            rw.at(1, i) = q;
+        } else {
+            C[base + i] = p;
+            C[NN + base + i] = q;
+        }
+    }
+    if (sb >= 0) {
+        __syncthreads();
+        rw.start(C, tab);
     }
 }
 
-// out[b] += sum |field|^2 of solve b's field at X + b*2*nn + off (FP64).
-__global__ void k_abs2_sum_b(const float2 *__restrict__ X, int nn, int off, double *out) {
-    const float2 *A = X + (size_t)blockIdx.y * 2 * nn + off;
+// out[b] += sum |field|^2 of solve b's field at X + b*stride (FP64).
+__global__ void k_abs2_sum_b(const float2 *__restrict__ X, int nn, size_t stride, double *out) {
+    const float2 *A = X + blockIdx.y * stride;
     double a[1] = {0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
         const float2 v = A[i];
@@ -167,22 +338,83 @@ cudaError_t launch_th_coef_table(const float *NP, const float *NS, const float *
     return cudaGetLastError();
 }
 
-cudaError_t launch_th_rk4_pair(float2 *X, float2 *save_w, float2 *save_x, const float4 *coef, int nn, int K, int sp,
-                               int sn, const InstDesc *d, int solves, cudaStream_t st) {
-    if (sp >= K || sn >= K) return cudaErrorInvalidValue;
-    k_th_rk4_pair<<<grid_b(nn, solves), 256, 0, st>>>(X, save_w, save_x, coef, nn, K, sp, sn, d);
-    return cudaGetLastError();
+// Row pass shape by the number of shape-0 blocks: us per z step, forward / gradient with 10
+// checkpoints, of shape 0, 1, 2 (GB300, 40 steps):
+//    < 1 per SM    64^2 x 4    6.6/14.8   6.0/13.2   5.4/11.7     256^2 x 2   12.5/31.6  10.7/27.7  10.1/27.6
+//    < 2 per SM   128^2 x 16  15.3/38.4  13.6/35.5  15.3/39.6     256^2 x 4   15.3/38.6  13.8/36.5  15.1/40.2
+//    more          64^2 x 64  12.8/32.2  13.4/34.4  12.5/34.1     256^2 x 8   21.1/58.4  22.2/62.6  24.4/69.9
+template <int N>
+static int row_shape(int solves, int sms) {
+    const int blocks = solves * ThRowShape<N, 0>::BPI;
+    return blocks < sms ? 2 : blocks < 2 * sms ? 1 : 0;
 }
 
-cudaError_t launch_th_vjp_pair(const float2 *Xa, const float2 *Wb, float2 *cot, const float4 *coef, int nn, int K,
-                               int sa, int sb, const InstDesc *d, int solves, cudaStream_t st) {
+template <int N, int SHAPE>
+static cudaError_t launch_rows_fwd_s(float2 *A, const float2 *inP, const float2 *inS, size_t stride, float2 *save_w,
+                                     float2 *save_x, float2 *out, const float4 *coef, int K, int sp, int sn,
+                                     const InstDesc *d, int solves, cudaStream_t st) {
+    using Sh = ThRowShape<N, SHAPE>;
+    return launch_dependent(k_th_rows_fwd<N, SHAPE>, dim3(Sh::BPI, solves), Sh::TPB, st, A, inP, inS, stride, save_w,
+                            save_x, out, coef, K, sp, sn, d);
+}
+
+template <int N>
+static cudaError_t launch_rows_fwd_t(float2 *A, const float2 *inP, const float2 *inS, size_t stride, float2 *save_w,
+                                     float2 *save_x, float2 *out, const float4 *coef, int K, int sp, int sn,
+                                     const InstDesc *d, int solves, int sms, cudaStream_t st) {
+    const int shape = row_shape<N>(solves, sms);
+    auto launch = shape == 0   ? launch_rows_fwd_s<N, 0>
+                  : shape == 1 ? launch_rows_fwd_s<N, 1>
+                               : launch_rows_fwd_s<N, 2>;
+    return launch(A, inP, inS, stride, save_w, save_x, out, coef, K, sp, sn, d, solves, st);
+}
+
+template <int N, int SHAPE>
+static cudaError_t launch_rows_bwd_s(float2 *C, const float2 *Xa, const float2 *Wb, const float4 *coef, int K, int sa,
+                                     int sb, const InstDesc *d, int solves, cudaStream_t st) {
+    using Sh = ThRowShape<N, SHAPE>;
+    return launch_dependent(k_th_rows_bwd<N, SHAPE>, dim3(Sh::BPI, solves), Sh::TPB, st, C, Xa, Wb, coef, K, sa, sb, d);
+}
+
+template <int N>
+static cudaError_t launch_rows_bwd_t(float2 *C, const float2 *Xa, const float2 *Wb, const float4 *coef, int K, int sa,
+                                     int sb, const InstDesc *d, int solves, int sms, cudaStream_t st) {
+    const int shape = row_shape<N>(solves, sms);
+    auto launch = shape == 0   ? launch_rows_bwd_s<N, 0>
+                  : shape == 1 ? launch_rows_bwd_s<N, 1>
+                               : launch_rows_bwd_s<N, 2>;
+    return launch(C, Xa, Wb, coef, K, sa, sb, d, solves, st);
+}
+
+cudaError_t launch_th_rows_fwd(int n, float2 *A, const float2 *inP, const float2 *inS, size_t stride, float2 *save_w,
+                               float2 *save_x, float2 *out, const float4 *coef, int K, int sp, int sn,
+                               const InstDesc *d, int solves, int sms, cudaStream_t st) {
+    if (sp >= K || sn >= K || (sp < 0 && !inP)) return cudaErrorInvalidValue;
+    switch (n) {
+        case 16: return launch_rows_fwd_t<16>(A, inP, inS, stride, save_w, save_x, out, coef, K, sp, sn, d, solves, sms, st);
+        case 32: return launch_rows_fwd_t<32>(A, inP, inS, stride, save_w, save_x, out, coef, K, sp, sn, d, solves, sms, st);
+        case 64: return launch_rows_fwd_t<64>(A, inP, inS, stride, save_w, save_x, out, coef, K, sp, sn, d, solves, sms, st);
+        case 128: return launch_rows_fwd_t<128>(A, inP, inS, stride, save_w, save_x, out, coef, K, sp, sn, d, solves, sms, st);
+        case 256: return launch_rows_fwd_t<256>(A, inP, inS, stride, save_w, save_x, out, coef, K, sp, sn, d, solves, sms, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_th_rows_bwd(int n, float2 *C, const float2 *Xa, const float2 *Wb, const float4 *coef, int K, int sa,
+                               int sb, const InstDesc *d, int solves, int sms, cudaStream_t st) {
     if (sa >= K || sb >= K || (sa >= 0 && !Xa) || (sb >= 0 && !Wb)) return cudaErrorInvalidValue;
-    k_th_vjp_pair<<<grid_b(nn, solves), 256, 0, st>>>(Xa, Wb, cot, coef, nn, K, sa, sb, d);
-    return cudaGetLastError();
+    switch (n) {
+        case 16: return launch_rows_bwd_t<16>(C, Xa, Wb, coef, K, sa, sb, d, solves, sms, st);
+        case 32: return launch_rows_bwd_t<32>(C, Xa, Wb, coef, K, sa, sb, d, solves, sms, st);
+        case 64: return launch_rows_bwd_t<64>(C, Xa, Wb, coef, K, sa, sb, d, solves, sms, st);
+        case 128: return launch_rows_bwd_t<128>(C, Xa, Wb, coef, K, sa, sb, d, solves, sms, st);
+        case 256: return launch_rows_bwd_t<256>(C, Xa, Wb, coef, K, sa, sb, d, solves, sms, st);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
-cudaError_t launch_abs2_sum_b(const float2 *X, int nn, int off, double *out, int solves, cudaStream_t st) {
-    k_abs2_sum_b<<<grid_b(nn, solves), 256, 0, st>>>(X, nn, off, out);
+cudaError_t launch_abs2_sum_b(const float2 *X, int nn, size_t stride, double *out, int solves, cudaStream_t st) {
+    k_abs2_sum_b<<<grid_b(nn, solves), 256, 0, st>>>(X, nn, stride, out);
     return cudaGetLastError();
 }
 

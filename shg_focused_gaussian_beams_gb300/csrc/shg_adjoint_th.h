@@ -17,14 +17,16 @@ class ThermalSolve;
 
 cudaError_t launch_th_coef_table(const float *NP, const float *NS, const float *DK, float4 *coef, int nn, int K,
                                  const ThermDesc &th, cudaStream_t st);
-// Fused step boundaries: forward RK4 of step sp (second call; input saved to save_w), state
-// saved to save_x, RK4 of step sn (first call); reverse RK4^T of step sa at Xa then of step
-// sb at Wb. A negative step index skips that half.
-cudaError_t launch_th_rk4_pair(float2 *X, float2 *save_w, float2 *save_x, const float4 *coef, int nn, int K, int sp,
-                               int sn, const InstDesc *d, int solves, cudaStream_t st);
-cudaError_t launch_th_vjp_pair(const float2 *Xa, const float2 *Wb, float2 *cot, const float4 *coef, int nn, int K,
-                               int sa, int sb, const InstDesc *d, int solves, cudaStream_t st);
-cudaError_t launch_abs2_sum_b(const float2 *X, int nn, int off, double *out, int solves, cudaStream_t st);
+// Fused row passes of a step boundary, every solve at once (see shg_adjoint_th.cu): forward (second
+// RK4 of step sp, its input saved to save_w, state saved to save_x, first RK4 of step sn) and
+// reverse (RK4^T of step sa at Xa, then of step sb at Wb). A negative step index skips that half;
+// sms: the device's SM count, by which the block shape is chosen.
+cudaError_t launch_th_rows_fwd(int n, float2 *A, const float2 *inP, const float2 *inS, size_t stride, float2 *save_w,
+                               float2 *save_x, float2 *out, const float4 *coef, int K, int sp, int sn,
+                               const InstDesc *d, int solves, int sms, cudaStream_t st);
+cudaError_t launch_th_rows_bwd(int n, float2 *C, const float2 *Xa, const float2 *Wb, const float4 *coef, int K, int sa,
+                               int sb, const InstDesc *d, int solves, int sms, cudaStream_t st);
+cudaError_t launch_abs2_sum_b(const float2 *X, int nn, size_t stride, double *out, int solves, cudaStream_t st);
 cudaError_t launch_seed_b(const float2 *X, float2 *cot, int nn, const double *seed, int solves, cudaStream_t st);
 
 // `count` solves on one NX = NY grid, each with its own fixed temperature field. Solve i's
@@ -57,7 +59,7 @@ class ThermalGradBatch {
     void drop_graphs();
 
     shg_config cfg_{};
-    int n_ = 0, nz_ = 0, K_ = 0, count_ = 0;
+    int n_ = 0, nz_ = 0, K_ = 0, count_ = 0, sms_ = 0;
     size_t nn_ = 0, tsize_ = 0;
     std::unique_ptr<ThermalSolve> ts_;
     // fixed per solve

@@ -71,6 +71,7 @@ int ThermalGradBatch::create(const shg_config &cfg, int count) {
     nn_ = (size_t)n_ * n_;
     tsize_ = nn_ * nz_;
     TG_CUDA(cudaSetDevice(cfg.device));
+    TG_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, cfg.device));
     TG_TRY(ensure_twiddles(cfg.device));
     const size_t c = (size_t)count;
     TG_TRY(device_fits(c * (tsize_ * sizeof(float) + (size_t)K_ * nn_ * sizeof(float4) + 3 * nn_ * sizeof(float2)),
@@ -214,22 +215,25 @@ int ThermalGradBatch::enqueue(bool grad, int L, int nseg, bool store_all, cudaSt
     int &nl = launches_;
     nl = 0;
     TG_CUDA(cudaMemsetAsync(sums_, 0, 2 * (size_t)B * sizeof(double), st));
-    TG_CUDA(cudaMemcpy2DAsync(X_, 2 * nn_ * sizeof(float2), in_, nn_ * sizeof(float2), nn_ * sizeof(float2), B,
-                              cudaMemcpyDeviceToDevice, st));
-    TG_CUDA(cudaMemset2DAsync(X_ + nn_, 2 * nn_ * sizeof(float2), 0, nn_ * sizeof(float2), B, st));
-    TG_CUDA(launch_abs2_sum_b(X_, nn, 0, sums_ + B, B, st));
+    TG_CUDA(launch_abs2_sum_b(in_, nn, nn_, sums_ + B, B, st));
     ++nl;
-    auto diffraction = [&](float2 *A, int mode, cudaStream_t q) -> int {
-        TG_CUDA(launch_dft_rows(n, +1, A, A, q, 2 * B));
-        TG_CUDA(launch_colpass(n, mode, A, nullptr, d_desc_, nullptr, q, B));
-        TG_CUDA(launch_dft_rows(n, -1, A, A, q, 2 * B));
-        nl += 3;
+    // between two row passes: the y transforms and the propagator
+    auto columns = [&](float2 *A, int mode, cudaStream_t q) -> int {
+        TG_CUDA(launch_colpass(n, mode, A, nullptr, d_desc_, nullptr, q, B, true));
+        ++nl;
         return SHG_OK;
     };
-    // Step boundary s (0 <= s <= K) of the forward march on X_: second RK4 of step s-1
-    // (input W_{s-1} to save_w), X_s to save_x, first RK4 of step s; one pass per boundary.
-    auto boundary = [&](int s, int s_end, float2 *save_w, float2 *save_x, cudaStream_t q) -> int {
-        TG_CUDA(launch_th_rk4_pair(X_, save_w, save_x, coef_, nn, K, s - 1, s < s_end ? s : -1, d_desc_, B, q));
+    // Step boundary s (s > 0) of the forward march on X_: second RK4 of step s-1 (input W_{s-1}
+    // to save_w), X_s to save_x, and with s < s_end the first RK4 of step s, else X_s to out.
+    auto boundary = [&](int s, int s_end, float2 *save_w, float2 *save_x, float2 *out, cudaStream_t q) -> int {
+        TG_CUDA(launch_th_rows_fwd(n, X_, nullptr, nullptr, 0, save_w, save_x, out, coef_, K, s - 1, s < s_end ? s : -1,
+                                   d_desc_, B, sms_, q));
+        ++nl;
+        return SHG_OK;
+    };
+    // Boundary s at the start of a march: the state from (P, S), `stride` apart.
+    auto enter = [&](int s, const float2 *P, const float2 *S, size_t stride, float2 *save_x, cudaStream_t q) -> int {
+        TG_CUDA(launch_th_rows_fwd(n, X_, P, S, stride, nullptr, save_x, nullptr, coef_, K, -1, s, d_desc_, B, sms_, q));
         ++nl;
         return SHG_OK;
     };
@@ -251,47 +255,44 @@ int ThermalGradBatch::enqueue(bool grad, int L, int nseg, bool store_all, cudaSt
         if (store_all) return Ws_ + (size_t)s * sz;
         return stored(s / L) ? Ws_ + slot_set(s / L) + (size_t)(s % L) * sz : nullptr;
     };
-    TG_TRY(boundary(0, K, nullptr, save_x(0), st));
+    TG_TRY(enter(0, in_, nullptr, nn_, save_x(0), st));
     for (int s = 0; s < K; ++s) {
-        TG_TRY(diffraction(X_, 0, st));
-        TG_TRY(boundary(s + 1, K, save_w(s), save_x(s + 1), st));
+        TG_TRY(columns(X_, 0, st));
+        TG_TRY(boundary(s + 1, K, save_w(s), save_x(s + 1), s + 1 < K ? nullptr : X_, st));
     }
-    TG_CUDA(launch_abs2_sum_b(X_, nn, nn, sums_, B, st));
+    TG_CUDA(launch_abs2_sum_b(X_ + nn_, nn, 2 * nn_, sums_, B, st));
     ++nl;
     if (!grad) return SHG_OK;
     TG_CUDA(launch_seed_b(X_, cot_, nn, seed_, B, st));
     ++nl;
-    // reverse sweep of steps [s0, s1) on `q` with the states X_s, W_s of those steps at
-    // Xs, Ws (slot s - s0): RK4^T at W_{s1-1}; then per step s the adjoint diffraction and
-    // one pass with RK4^T at X_s and at W_{s-1}
-    auto backward = [&](int s0, int s1, const float2 *Xs, const float2 *Ws, cudaStream_t q) -> int {
-        TG_CUDA(launch_th_vjp_pair(nullptr, Ws + (size_t)(s1 - 1 - s0) * sz, cot_, coef_, nn, K, -1, s1 - 1, d_desc_,
-                                   B, q));
+    // Reverse sweep: RK4^T at W of the last step, then per step the adjoint diffraction and one
+    // pass with RK4^T at X_s and at W_{s-1}.
+    auto reverse = [&](const float2 *Xs, const float2 *Ws, int sa, int sb) -> int {
+        TG_CUDA(launch_th_rows_bwd(n, cot_, Xs, Ws, coef_, K, sa, sb, d_desc_, B, sms_, st));
         ++nl;
-        for (int s = s1 - 1; s >= s0; --s) {
-            TG_TRY(diffraction(cot_, 2, q));
-            const size_t j = (size_t)(s - s0) * sz;
-            const bool more = s - 1 >= s0;
-            TG_CUDA(launch_th_vjp_pair(Xs + j, more ? Ws + j - sz : nullptr, cot_, coef_, nn, K, s, more ? s - 1 : -1,
-                                       d_desc_, B, q));
-            ++nl;
-        }
         return SHG_OK;
     };
-    if (store_all) return backward(0, K, Xs_, Ws_, st);
+    if (store_all) {
+        TG_TRY(reverse(nullptr, Ws_ + (size_t)(K - 1) * sz, -1, K - 1));
+        for (int s = K - 1; s >= 0; --s) {
+            TG_TRY(columns(cot_, 2, st));
+            TG_TRY(reverse(Xs_ + (size_t)s * sz, s > 0 ? Ws_ + (size_t)(s - 1) * sz : nullptr, s, s - 1));
+        }
+        return SHG_OK;
+    }
     // The other segments are replayed from their checkpoints on the side branch into their
     // slot set (X_ is the replay's working state; the reverse sweep works on cot_), so the
-    // replay of segment seg-1 runs while segment seg is reversed on `st`.
+    // replay of segment seg-1 runs while segment seg is reversed on `st`. X_s0 is the checkpoint
+    // itself.
     auto replay = [&](int seg, cudaStream_t q) -> int {
         const int s0 = seg * L, s1 = std::min(K, s0 + L);
+        const float2 *c = ck_ + (size_t)seg * sz;
         float2 *Xs = Xs_ + slot_set(seg), *Ws = Ws_ + slot_set(seg);
-        TG_CUDA(cudaMemcpyAsync(X_, ck_ + (size_t)seg * sz, sz * sizeof(float2), cudaMemcpyDeviceToDevice, q));
-        TG_CUDA(launch_th_rk4_pair(X_, nullptr, Xs, coef_, nn, K, -1, s0, d_desc_, B, q));
-        ++nl;
+        TG_TRY(enter(s0, c, c + nn_, 2 * nn_, nullptr, q));
         for (int s = s0; s < s1; ++s) {
-            TG_TRY(diffraction(X_, 0, q));
+            TG_TRY(columns(X_, 0, q));
             const size_t j = (size_t)(s - s0) * sz;
-            TG_TRY(boundary(s + 1, s1, Ws + j, s + 1 < s1 ? Xs + j + sz : nullptr, q));
+            TG_TRY(boundary(s + 1, s1, Ws + j, s + 1 < s1 ? Xs + j + sz : nullptr, nullptr, q));
         }
         return SHG_OK;
     };
@@ -301,18 +302,28 @@ int ThermalGradBatch::enqueue(bool grad, int L, int nseg, bool store_all, cudaSt
         TG_CUDA(cudaStreamWaitEvent(b, ev_, 0));
         return SHG_OK;
     };
+    auto state_x = [&](int s) -> const float2 * {  // X_s as the reverse sweep reads it
+        const int seg = s / L;
+        return !stored(seg) && s % L == 0 ? ck_ + (size_t)seg * sz : Xs_ + slot_set(seg) + (size_t)(s % L) * sz;
+    };
+    auto state_w = [&](int s) -> const float2 * { return Ws_ + slot_set(s / L) + (size_t)(s % L) * sz; };
     for (int seg = nseg - 1; seg >= 0; --seg) {
-        if (!stored(seg)) TG_TRY(join(side_, st));  // replay(seg) done
-        // replay(seg-1) reuses the slot set of segment seg+1, whose reverse sweep st finished
-        // (and the seed has read the forward's final X_ before the first replay)
+        // the pass that enters segment seg reads the last states of its replay (and, of segment
+        // seg+1, whose slot set the replay of seg-1 reuses after it, X of the first step)
+        if (!stored(seg)) TG_TRY(join(side_, st));
+        const int s0 = seg * L, s1 = std::min(K, s0 + L);
+        TG_TRY(reverse(s1 < K ? state_x(s1) : nullptr, state_w(s1 - 1), s1 < K ? s1 : -1, s1 - 1));
+        // (the seed has read the forward's final X_ before the first replay)
         if (seg >= 1 && !stored(seg - 1)) {
             TG_TRY(join(st, side_));
             TG_TRY(replay(seg - 1, side_));
         }
-        const int s0 = seg * L, s1 = std::min(K, s0 + L);
-        TG_TRY(backward(s0, s1, Xs_ + slot_set(seg), Ws_ + slot_set(seg), st));
+        for (int s = s1 - 1; s >= s0; --s) {
+            TG_TRY(columns(cot_, 2, st));
+            if (s > s0) TG_TRY(reverse(state_x(s), state_w(s - 1), s, s - 1));
+        }
     }
-    return SHG_OK;
+    return reverse(state_x(0), nullptr, 0, -1);
 }
 
 int ThermalGradBatch::finish(double *p_sh, double *p_in, cudaStream_t st) {

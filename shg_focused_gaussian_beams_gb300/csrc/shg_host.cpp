@@ -210,7 +210,8 @@ int ensure_twiddles(int device) {
     for (const float2 *addr : {twiddle_symbol_address_march(), twiddle_symbol_address_thermal(),
                                twiddle_symbol_address_adjoint(), twiddle_symbol_address_resident(),
                                twiddle_symbol_address_resident128(), twiddle_symbol_address_resident256(),
-                               twiddle_symbol_address_cluster_pt(), twiddle_symbol_address_group()}) {
+                               twiddle_symbol_address_cluster_pt(), twiddle_symbol_address_group(),
+                               twiddle_symbol_address_adjoint_th()}) {
         void *p = const_cast<float2 *>(addr);
         if (!p) {
             set_error("twiddle table symbol unavailable");
@@ -1920,7 +1921,8 @@ int shg_check_status(int *enabled, int *site, long long *value) {
     unsigned long long first = 0;
     for (auto take : {check_word_take_march, check_word_take_resident64, check_word_take_resident128,
                       check_word_take_resident256, check_word_take_cluster_pt, check_word_take_thermal,
-                      check_word_take_heat_tma, check_word_take_heat_block, check_word_take_group, check_word_take_adjoint}) {
+                      check_word_take_heat_tma, check_word_take_heat_block, check_word_take_group, check_word_take_adjoint,
+                      check_word_take_adjoint_th}) {
         const unsigned long long w = take();
         if (w == ~0ull) {
             set_error("shg_check_status: status word unreadable");

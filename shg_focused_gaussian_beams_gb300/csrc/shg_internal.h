@@ -31,6 +31,7 @@ const float2 *twiddle_symbol_address_resident128();
 const float2 *twiddle_symbol_address_resident256();
 const float2 *twiddle_symbol_address_cluster_pt();
 const float2 *twiddle_symbol_address_group();
+const float2 *twiddle_symbol_address_adjoint_th();
 
 // Check build (shg_check.cuh): each kernel translation unit's first failed check, read and
 // cleared (0: none; ~0: unreadable); always 0 in other builds.
@@ -43,6 +44,7 @@ unsigned long long check_word_take_thermal();
 unsigned long long check_word_take_heat_tma();
 unsigned long long check_word_take_heat_block();
 unsigned long long check_word_take_group();
+unsigned long long check_word_take_adjoint_th();
 unsigned long long check_word_take_adjoint();
 cudaError_t launch_check_selftest(long long value);
 
@@ -87,7 +89,6 @@ constexpr int kMaxGroups = 512, kGroupWords = 1 + 2 * kMaxGroups;
 cudaError_t launch_group(int n, const InstDesc *inst, const int *list, int njobs, unsigned *words, int *err,
                          cudaStream_t st, int *max_groups = nullptr);
 cudaError_t launch_dft2d(int n, int sign, const float2 *in, float2 *out, cudaStream_t st);
-cudaError_t launch_dft_rows(int n, int sign, const float2 *in, float2 *out, cudaStream_t st, int fields = 1);
 
 // shg_thermal.cu
 struct HeatCoef;

@@ -30,9 +30,6 @@ struct InstDesc {
     float hp;               // 0.5*alpha_p
     float tpa0, tpa1;       // 0.5*alpha_s, 0.25*beta_s*C*EPS0*n_s
     float kp, ks;           // pi*dQ/(n_p*lp), 0.5*pi*dQ/(n_s*ls)
-    float sp, ss;           // scales of the marched fields (march_scales): p = sp P, s = ss S
-    float isp, iss;         // 1/sp, 1/ss
-    float tpa1s;            // tpa1 / ss^2
     float dk;               // phase mismatch (PhaseMatching.h:57-70), float
     // Gaussian pump (Efields.h:74-104): exact float operands of the reference.
     float uX, uY, dx, dy;
@@ -45,6 +42,9 @@ struct InstDesc {
     float linp, lins;       // 2*PI*dfX*tan(rho)
     float mdz;              // -dz
     float inv_nn;           // 1/(n*n), exact for power-of-two n
+    float sp, ss;           // scales of the marched fields (march_scales): p = sp P, s = ss S
+    float isp, iss;         // 1/sp, 1/ss
+    float tpa1s;            // tpa1 / ss^2
 };
 
 // dA/dz of Solver.h:65-83 for one point, with the per-slice constants folded:

@@ -101,9 +101,9 @@ __device__ __forceinline__ ThCoef th_coef_k(float kp, float ks, float tpa1, floa
 // The same with the temperature field held fixed (the batched gradient): the phases are
 // DKint dz (1 + inc/(s+1)), so one sincosf at inc = 0 and two rotations by the angle
 // d = DKint dz / (4 (s+1)), a quarter step of the mean mismatch, serve the four stages. With
-// three sincosf and three divisions per RK4 call the constants were a third of the pointwise
-// passes: k_th_rk4_pair 25.4 -> 22.6 us, k_th_vjp_pair 36.5 -> 31.5 us at 16 x 256 x 256 points
-// (of which 14 us are the bytes that the first one moves, at HBM rate).
+// three sincosf and three divisions per RK4 call the constants were a third of the boundary
+// passes' pointwise work (at 16 x 256 x 256 points, in passes of their own: forward 25.4 -> 22.6 us,
+// reverse 36.5 -> 31.5 us).
 __device__ __forceinline__ ThCoef th_coef_fixed(float kp, float ks, float tpa1, float dkint, int s, float dz) {
     ThCoef r;
     const float ph0 = dkint * dz, d = ph0 * __fdividef(0.25f, (float)(s + 1));
