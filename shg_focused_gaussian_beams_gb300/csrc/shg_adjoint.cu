@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(TC * LineShape<N>::G) k_colpass(float2 *A0, fl
                                                              const InstDesc *__restrict__ dd, double *acc0) {
     constexpr int G = LineShape<N>::G, E = N / G;
     __shared__ float2 scratch[TC * E * G];
+    __shared__ float stage[MODE == 1 ? TC * G : 1];
     const float2 *__restrict__ tab = g_twiddle + N;
     const int f = blockIdx.y;
     const InstDesc &d = dd[f >> 1];
@@ -91,10 +92,11 @@ __global__ void __launch_bounds__(TC * LineShape<N>::G) k_colpass(float2 *A0, fl
             v[r] = c_mulc(v[r], h);                   // conj(H') X
         }
     }
+    if (MODE == 1) stage[threadIdx.x] = a;  // read after the transform's block barriers
     fft_spec_to_nat<N, G, -1, true, TC, G>(v, t, scratch + c, tab);
 #pragma unroll
     for (int j = 0; j < E; ++j) A[(size_t)(t + G * j) * N + x] = v[j];
-    if (MODE == 1) block_sum_f2d(&a, 1, acc);
+    if (MODE == 1 && threadIdx.x < 32) staged_sums(stage, 1, 0, 1, [&](int) { return acc; });
 }
 
 // ---------------------------------------------------------------------------------------
@@ -168,6 +170,7 @@ __global__ void __launch_bounds__(AdjRowShape<N>::TPB)
     using Cx = AdjRowCtx<N>;
     __shared__ float2 scratch[2 * Cx::LPB * Cx::SC];
     __shared__ float2 lines[2][Cx::LPB * N];
+    __shared__ float stage[10 * Cx::Sh::TPB];  // the sums of both transposed RK4 calls
     const InstDesc &d = *dd;
     if (!SHG_REQUIRE(d.n == N && (!finish || (s + 1 >= 0 && s + 1 < d.nz)) && (!start || (s >= 0 && s < d.nz)),
                      kChkAdjoint, s))
@@ -198,18 +201,29 @@ __global__ void __launch_bounds__(AdjRowShape<N>::TPB)
         cp = C[cx.i2];
         cs = C[nn + cx.i2];
     }
+    const int tid = threadIdx.x;
+    if (finish)
+#pragma unroll
+        for (int j = 0; j < 5; ++j) stage[j * Cx::Sh::TPB + tid] = a1[j];
     if (start) {
         rk4_vjp_point(wp, ws, cp, cs, d.stepc[s], hp, t0, t1, w6, a2);
         lines[0][cx.lx] = cp;  // each point thread rewrites only the entry it read
         lines[1][cx.lx] = cs;
-        __syncthreads();
-        cx.start(C, tab);
+#pragma unroll
+        for (int j = 0; j < 5; ++j) stage[(5 + j) * Cx::Sh::TPB + tid] = a2[j];
     } else {
         C[cx.i2] = cp;
         C[nn + cx.i2] = cs;
     }
-    if (finish) block_sum_f2d(a1, 5, acc_fin);
-    if (start) block_sum_f2d(a2, 5, acc_start);
+    __syncthreads();
+    if (start) cx.start(C, tab);
+    // The warps that do not transform sum meanwhile (behind the transform these sums, 16 dependent
+    // FP64 adds and a shuffle tree per call, made the pass 10.2 us instead of 8.8). Quantities 0..4 of the call
+    // at X_{s+1}, then 0..4 of the call at W_s.
+    const int w = (tid >> 5) - Cx::Sh::W0, q0 = finish ? 0 : 5;
+    if (w >= 0)
+        staged_sums(stage + q0 * Cx::Sh::TPB, (finish ? 5 : 0) + (start ? 5 : 0), w, Cx::Sh::NW,
+                    [&](int j) { return q0 + j < 5 ? acc_fin + j : acc_start + (q0 + j - 5); });
 }
 
 // sum |S|^2 of a field (FP64).

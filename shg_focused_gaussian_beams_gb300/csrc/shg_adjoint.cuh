@@ -45,20 +45,18 @@ __device__ __forceinline__ void block_sum_doubles(double *v, int k, double *dst)
     }
 }
 
-// Adds the block's k per-thread FP32 partial sums (k <= 5, blockDim <= 512) to dst[0..k)
-// in FP64: the partials are staged in shared memory and warp j sums quantity j in double,
-// so a thread converts 512/32 values of one quantity instead of reducing five doubles.
-__device__ __forceinline__ void block_sum_f2d(const float *v, int k, double *dst) {
-    __shared__ float stage[5][512];
-    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, nt = blockDim.x;
-    __syncthreads();  // earlier users of the stage are done
-    for (int j = 0; j < k; ++j) stage[j][tid] = v[j];
-    __syncthreads();
-    if (w < k) {
+// Sums of per-thread FP32 values over the block in FP64: a thread stores quantity j's value in
+// stage[j * blockDim + tid]; after a block barrier warp `w` of `nw` (any warps of the block) sums
+// quantities w, w + nw, ... < k and adds them to dst_of(j) with one FP64 atomic each, so a lane
+// converts blockDim / 32 values of one quantity instead of reducing them all.
+template <class Dst>
+__device__ __forceinline__ void staged_sums(const float *stage, int k, int w, int nw, Dst dst_of) {
+    const int l = threadIdx.x & 31, nt = blockDim.x;
+    for (int j = w; j < k; j += nw) {
         double a = 0.0;
-        for (int i = l; i < nt; i += 32) a += (double)stage[w][i];
+        for (int i = l; i < nt; i += 32) a += (double)stage[j * nt + i];
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (l == 0 && a != 0.0) atomicAdd(dst + w, a);
+        if (l == 0 && a != 0.0) atomicAdd(dst_of(j), a);
     }
 }
 
@@ -143,7 +141,7 @@ __device__ __forceinline__ void rk4_vjp_point(float2 P, float2 S, float2 &cP, fl
 }
 
 // Fused row passes for one solve, one thread per point (block = LPB lines x N threads; the
-// x-transforms of the pump and SH lines run on two groups of LPB * G threads). Between two
+// x-transforms of the pump and SH lines run on two groups of LPB LW lanes). Between two
 // column passes a row pass finishes one diffraction along x, applies the pointwise RK4 (or
 // RK4^T) work of the step boundary, and starts the next diffraction along x, so a z-step
 // costs one row and one column launch. The working state A / cotangent C holds the pump
@@ -155,7 +153,8 @@ struct AdjRowShape {
     static constexpr int LPB = (512 / N < N) ? 512 / N : N;
     static constexpr int TPB = LPB * N;
     static constexpr int BPI = N / LPB;
-    static constexpr int FT = LPB * G;  // transform threads per field
+    static constexpr int LW = RowLanes<N, false>::LW, FT = LPB * LW;  // transform lanes per field
+    static constexpr int W0 = 2 * FT < TPB ? 2 * FT / 32 : 0, NW = TPB / 32 - W0;  // warps free of them, if any
     static_assert(FT % 32 == 0 && 2 * FT <= TPB && N % LPB == 0, "transform threads fill whole warps");
 };
 
@@ -163,9 +162,8 @@ struct AdjRowShape {
 template <int N>
 struct AdjRowCtx {
     using Sh = AdjRowShape<N>;
-    static constexpr int G = Sh::G, E = N / G, LPB = Sh::LPB, FT = Sh::FT, SC = LineScratch<N, G>::SIZE;
+    static constexpr int G = Sh::G, LW = Sh::LW, LPB = Sh::LPB, FT = Sh::FT, SC = LineScratch<N, G>::SIZE;
     float2 *fline, *fsc;  // transform role: this thread's line buffer and FFT scratch
-    int t;
     bool xf;
     size_t frow;          // offset of the transformed row in A (field included)
     size_t i2;            // point role: index of the point in one field
@@ -173,8 +171,7 @@ struct AdjRowCtx {
     __device__ AdjRowCtx(float2 (*lines)[LPB * N], float2 *scratch) {
         const int tid = threadIdx.x, line0 = blockIdx.x * LPB;
         xf = tid < 2 * FT;
-        const int f = (tid / FT) & 1, fl = (tid % FT) / G;
-        t = tid % G;
+        const int f = (tid / FT) & 1, fl = (tid % FT) / LW;
         fline = lines[f] + fl * N;
         fsc = scratch + (size_t)(f * LPB + fl) * SC;
         frow = (size_t)f * N * N + (size_t)(line0 + fl) * N;
@@ -182,27 +179,16 @@ struct AdjRowCtx {
         i2 = (size_t)(line0 + l) * N + x;
         lx = l * N + x;
     }
+    __device__ RowLanes<N, false> split(const float2 *tab) const {
+        return RowLanes<N, false>(threadIdx.x % LW, fline, fsc, tab);
+    }
     // rows of A (natural frequency order) -> line buffers in real space (natural x order)
-    __device__ void finish(const float2 *A, const float2 *tab) {
-        if (xf) {
-            float2 v[E];
-#pragma unroll
-            for (int j = 0; j < E; ++j) v[j] = A[frow + t + G * j];
-            fft_nat_to_spec<N, G, -1>(v, t, fsc, tab);
-#pragma unroll
-            for (int r = 0; r < E; ++r) fline[spec_index<N, G>(t, r)] = v[r];
-        }
+    __device__ void finish(const float2 *A, const float2 *tab) const {
+        if (xf) split(tab).template to_spec<-1>(A + frow, fline);
     }
     // line buffers (real space) -> rows of A in natural frequency order
-    __device__ void start(float2 *A, const float2 *tab) {
-        if (xf) {
-            float2 v[E];
-#pragma unroll
-            for (int r = 0; r < E; ++r) v[r] = fline[spec_index<N, G>(t, r)];
-            fft_spec_to_nat<N, G, +1>(v, t, fsc, tab);
-#pragma unroll
-            for (int j = 0; j < E; ++j) A[frow + t + G * j] = v[j];
-        }
+    __device__ void start(float2 *A, const float2 *tab) const {
+        if (xf) split(tab).start(A + frow);
     }
 };
 

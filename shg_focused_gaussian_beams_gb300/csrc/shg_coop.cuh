@@ -55,28 +55,68 @@ struct CoopShape {
     static constexpr int G = LineShape<N>::G, E = N / G;
     static constexpr int LPB = (512 / N < N) ? 512 / N : N;  // lines per row unit
     static constexpr int TPB = LPB * N;                     // one thread per point of a unit
-    static constexpr int TC = 32 / G;                    // columns per column group (one warp)
+    static constexpr int TC = 32 / G;                    // columns per column group
     static constexpr int ROW_UNITS = N / LPB;            // groups of LPB lines
     static constexpr int COL_UNITS = 2 * (N / TC);       // column groups of both fields
-    static_assert(TC * G == 32, "a column group is one warp");
+    static constexpr bool SPLIT = RowLanes<N, true>::SPLIT;
+    static constexpr int GW = SPLIT ? 2 : 1;             // warps of a column group
+    static constexpr int OUT = E / GW;                   // spectrum values per thread
+    static_assert(TC * G == 32, "a column group is one warp, two of split lanes");
 };
 
-// cols_body with the column's propagator values already in registers.
-template <int N, int TC>
-__device__ __forceinline__ void cols_body_h(const InstDesc &d, int x, int f, int t, float2 *sc,
-                                            const float2 (&h)[N / LineShape<N>::G], const float2 *tab) {
-    constexpr int G = LineShape<N>::G, E = N / G;  // tab: the split's pair table in shared memory
-    float2 *F = f == 0 ? d.P : d.S;
-    constexpr size_t NN = (size_t)N * N;
-    float2 v[E];
+// Column group of a block: TC columns of one field on one warp, or split on two (warp h of the pair
+// computes the outputs 2 r + h; a named barrier of their own synchronises them). The columns'
+// propagator values stay in registers for the whole run. Block b of B holds groups b, b + B, ...
+template <int N>
+struct CoopColumn {
+    using C = CoopShape<N>;
+    static constexpr int G = C::G, E = C::E, TC = C::TC, OUT = C::OUT;
+    struct PairSync {
+        int id;
+        __device__ void operator()() const { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+    };
+    bool active;
+    int g, h, f, x, t;
+    __device__ CoopColumn(int block, int blocks, int groups) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        g = warp / C::GW;
+        h = warp % C::GW;
+        const int u = block + blocks * g;
+        active = g < groups && u < C::COL_UNITS;
+        f = u / (N / TC);
+        x = (u % (N / TC)) * TC + lane % TC;
+        t = lane / TC;
+    }
+    __device__ __forceinline__ void load(const InstDesc &d, float2 (&hp)[OUT]) const {
+        const float2 *H = f == 0 ? d.Hp : d.Hs;
+        if constexpr (C::SPLIT) split_hprop_load<N>(H, x, t, h, hp);
+        else hprop_load<N>(H, x, t, hp);
+    }
+    // scr: TC * N float2 per group; tab: the split's twiddle pairs in shared memory
+    __device__ __forceinline__ void run(const InstDesc &d, float2 *scr, const float2 (&hp)[OUT], const float2 *tab) const {
+        float2 *const F = f == 0 ? d.P : d.S, *const sc = scr + (size_t)g * TC * N + threadIdx.x % TC;
+        [[maybe_unused]] constexpr size_t NN = (size_t)N * N;
+        float2 v[E];
 #pragma unroll
-    for (int j = 0; j < E; ++j) v[j] = SHG_AT(F, (size_t)(t + G * j) * N + x, NN, kChkCoop);
-    fft_nat_to_spec<N, G, +1, false, TC, G, true>(v, t, sc, tab);
+        for (int j = 0; j < E; ++j) v[j] = SHG_AT(F, (size_t)(t + G * j) * N + x, NN, kChkCoop);
+        if constexpr (C::SPLIT) {
+            float2 o[OUT];
+            column_split<N, TC, true>(v, o, t, h, sc, tab, PairSync{g + 1},
+                                      [&](int r, float2 a) { return c_mul(a, hp[r]); });
 #pragma unroll
-    for (int r = 0; r < E; ++r) v[r] = c_mul(v[r], h[r]);
-    fft_spec_to_nat<N, G, -1, false, TC, G, true>(v, t, sc, tab);
+            for (int r = 0; r < OUT; ++r) {
+                const size_t y = SplitLine<N, G>::nat(t, h, r);
+                SHG_AT(F, y * N + x, NN, kChkCoop) = o[r];
+            }
+        } else {
+            fft_nat_to_spec<N, G, +1, false, TC, G, true>(v, t, sc, tab);
 #pragma unroll
-    for (int j = 0; j < E; ++j) SHG_AT(F, (size_t)(t + G * j) * N + x, NN, kChkCoop) = v[j];
-}
+            for (int r = 0; r < E; ++r) v[r] = c_mul(v[r], hp[r]);
+            fft_spec_to_nat<N, G, -1, false, TC, G, true>(v, t, sc, tab);
+#pragma unroll
+            for (int j = 0; j < E; ++j) SHG_AT(F, (size_t)(t + G * j) * N + x, NN, kChkCoop) = v[j];
+        }
+    }
+};
 
 }  // namespace shg

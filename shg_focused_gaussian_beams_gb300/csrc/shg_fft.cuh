@@ -244,6 +244,226 @@ __device__ __forceinline__ int spec_index(int t, int r) {
     return (t * Q + m) + E * k1;
 }
 
+// ---------------------------------------------------------------------------------------
+// Split transforms: a line on 2 G lanes, two per thread of the transforms above. Both lanes of a
+// pair (h = 0, 1) take thread t's inputs, and lane h computes the outputs 2 r + h: after the first
+// radix-2 stage, x_i +- x_{i+E/2}, the even and the odd outputs of an E-point DFT are DFTs that share
+// nothing. Every output passes through the same butterflies with the same roundings as in
+// dft_reg, so the results are the same bits; a lane executes about 0.55 of the instructions, which
+// is what a lone solve, whose SMs hold one or two transforming warps, takes its time for.
+
+// Outputs 2 r + h of the E-point DFT of v, r < E/2 (E <= 16). The lanes' stages differ in their
+// twiddles: lane 1's is w^(h 32 / len) further. Where dft_reg multiplies by w^8 = +-i or adds 8 to the
+// exponent, y is turned by +-i first (exact) and the rest is the same form; the remaining pairs of
+// exponents, (0, 4), (0, 2) and (4, 6), share the cosine or the sine form with per-lane constants
+// (of the trivial twiddle 1 and 0, whose products are exact).
+template <int E, int SIGN, int NV>
+__device__ __forceinline__ void dft_half(const float2 (&v)[NV], float2 (&o)[E / 2], int h) {
+    static_assert(E >= 4 && E <= 16 && NV >= E, "split DFT size");
+    constexpr int M = E / 2, LG = ilog2(M);
+    constexpr float sg = SIGN > 0 ? 1.0f : -1.0f;
+    const float s1 = h ? -1.0f : 1.0f;
+    float2 u[M];
+    sfor<M>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        u[bitrev(i, LG)] = make_float2(fmaf(s1, v[i + M].x, v[i].x), fmaf(s1, v[i + M].y, v[i].y));
+    });
+    sfor<LG>([&](auto S) {
+        constexpr int half = 1 << decltype(S)::value, len = 4 * half;  // dft_reg's stage of length len
+        sfor<M / 2>([&](auto B) {
+            constexpr int grp = decltype(B)::value / half, q = decltype(B)::value % half;
+            constexpr int a = grp * 2 * half + q, b = a + half;
+            constexpr int base = q * (64 / len), step = 32 / len;  // exponent of lane 0, further of lane 1
+            const float2 x = u[a];
+            float2 y = u[b];
+            if constexpr (base >= 8) y = make_float2(-sg * y.y, sg * y.x);
+            if constexpr (step == 8) {
+                y = h ? make_float2(-sg * y.y, sg * y.x) : y;
+                u[a] = c_add(x, y);
+                u[b] = c_sub(x, y);
+            } else if constexpr (base % 8 == 0) {
+                constexpr float c1 = W32::c[step], t1 = sg * TanPi16::t[step];
+                const float c = h ? c1 : 1.0f, tau = h ? t1 : 0.0f;
+                const float ux = fmaf(-tau, y.y, y.x), uy = fmaf(tau, y.x, y.y);
+                u[a] = make_float2(fmaf(c, ux, x.x), fmaf(c, uy, x.y));
+                u[b] = make_float2(fmaf(-c, ux, x.x), fmaf(-c, uy, x.y));
+            } else {
+                static_assert(base % 8 == 4 && step == 2, "exponents 4 and 6");
+                constexpr float c0 = sg * W32::s[4], c1 = sg * W32::s[4 + step];
+                constexpr float k0 = sg * TanPi16::t[4], k1 = sg * TanPi16::t[4 - step];
+                const float c = h ? c1 : c0, kap = h ? k1 : k0;
+                const float ux = fmaf(kap, y.x, -y.y), uy = fmaf(kap, y.y, y.x);
+                u[a] = make_float2(fmaf(c, ux, x.x), fmaf(c, uy, x.y));
+                u[b] = make_float2(fmaf(-c, ux, x.x), fmaf(-c, uy, x.y));
+            }
+        });
+    });
+    sfor<M>([&](auto I) { o[decltype(I)::value] = u[decltype(I)::value]; });
+}
+
+// Shapes of a split line: OUT values per lane after either transform; IN inputs per lane of the
+// spectral-to-natural one (both lanes need all where a thread holds one G-point DFT, and one DFT
+// each where it holds two).
+template <int N, int G>
+struct SplitLine {
+    static constexpr int E = N / G, Q = E / G, OUT = E / 2, IN = Q == 1 ? E : E / 2;
+    static_assert(E == Q * G && (Q == 1 || Q == 2), "split of a line");
+    // spectral index of output r of nat_to_spec / of input r of spec_to_nat; natural index of output r
+    __device__ static int spec(int t, int h, int r) { return Q == 1 ? t + E * (2 * r + h) : 2 * t + h + E * r; }
+    __device__ static int spec_in(int t, int h, int r) { return Q == 1 ? t + E * r : 2 * t + h + E * r; }
+    __device__ static int nat(int t, int h, int r) { return t + G * (2 * r + h); }
+};
+
+// fft_nat_to_spec on split lanes: v holds thread t's E inputs (index t + G j), o the outputs
+// (SplitLine::spec). sync: of the line's lanes. TS as for twiddle_mul.
+template <int N, int G, int SIGN, int STRIDE, int GP, bool TS, class Sync>
+__device__ __forceinline__ void fft_nat_to_spec_split(const float2 (&v)[N / G], float2 (&o)[N / G / 2], int t, int h,
+                                                      float2 *sc, const float2 *__restrict__ tab, Sync sync) {
+    using L = SplitLine<N, G>;
+    constexpr int E = L::E, M = E / 2;
+    dft_half<E, SIGN>(v, o, h);
+    const float2 *__restrict__ w = (TS ? tab : twiddle_split<N, G>(tab)) + 2 * t + h;
+#pragma unroll
+    for (int r = 0; r < M; ++r) {  // k2 = 2 r + h; the word of k2 = 0 holds 1
+        const float2 q = TS ? w[2 * r * G] : __ldg(w + 2 * r * G);
+        o[r] = c_mul(o[r], make_float2(q.x, SIGN > 0 ? -q.y : q.y));
+    }
+    sync();
+#pragma unroll
+    for (int r = 0; r < M; ++r) sc[((2 * r + h) * GP + t) * STRIDE] = o[r];
+    sync();
+    if constexpr (L::Q == 1) {
+        float2 g[G];
+#pragma unroll
+        for (int tt = 0; tt < G; ++tt) g[tt] = sc[(t * GP + tt) * STRIDE];
+        dft_half<G, SIGN>(g, o, h);
+    } else {
+#pragma unroll
+        for (int tt = 0; tt < G; ++tt) o[tt] = sc[((2 * t + h) * GP + tt) * STRIDE];
+        dft_reg<G, SIGN>(o);
+    }
+}
+
+// fft_spec_to_nat on split lanes: v holds the inputs SplitLine::spec_in, o the outputs
+// (SplitLine::nat).
+template <int N, int G, int SIGN, int STRIDE, int GP, bool TS, class Sync>
+__device__ __forceinline__ void fft_spec_to_nat_split(float2 (&v)[SplitLine<N, G>::IN], float2 (&o)[N / G / 2], int t,
+                                                      int h, float2 *sc, const float2 *__restrict__ tab, Sync sync) {
+    using L = SplitLine<N, G>;
+    constexpr int E = L::E;
+    if constexpr (L::Q == 1) {
+        dft_half<G, SIGN>(v, o, h);
+        // twiddles before the exchange: w^(tt k2) of tt = 2 r + h, k2 = t from thread t's own words
+        const float2 *__restrict__ w = (TS ? tab : twiddle_split<N, G>(tab)) + 2 * t + h;
+#pragma unroll
+        for (int r = 0; r < G / 2; ++r) {
+            const float2 q = TS ? w[2 * r * G] : __ldg(w + 2 * r * G);
+            o[r] = c_mul(o[r], make_float2(q.x, SIGN > 0 ? -q.y : q.y));
+        }
+        sync();
+#pragma unroll
+        for (int r = 0; r < G / 2; ++r) sc[(t * GP + 2 * r + h) * STRIDE] = o[r];
+        sync();
+#pragma unroll
+        for (int k2 = 0; k2 < E; ++k2) v[k2] = sc[(k2 * GP + t) * STRIDE];
+        dft_half<E, SIGN>(v, o, h);
+    } else {
+        dft_reg<G, SIGN>(v);
+        sync();
+#pragma unroll
+        for (int tt = 0; tt < G; ++tt) sc[((2 * t + h) * GP + tt) * STRIDE] = v[tt];
+        sync();
+        float2 a[E];
+#pragma unroll
+        for (int k2 = 0; k2 < E; ++k2) a[k2] = sc[(k2 * GP + t) * STRIDE];
+        twiddle_mul<N, G, SIGN, TS>(a, t, tab);
+        dft_half<E, SIGN>(a, o, h);
+    }
+}
+
+struct WarpSync {
+    __device__ void operator()() const { __syncwarp(); }
+};
+
+// One z step's column pass of a line on split lanes (t, h): backward transform of thread t's elements
+// v of the column, mid(r, value) on this lane's outputs (SplitLine::spec), forward transform to o
+// (SplitLine::nat). Column scratch: elements STRIDE apart.
+template <int N, int STRIDE, bool TS, class Sync, class Mid>
+__device__ __forceinline__ void column_split(const float2 (&v)[N / LineShape<N>::G],
+                                             float2 (&o)[N / LineShape<N>::G / 2], int t, int h, float2 *sc,
+                                             const float2 *__restrict__ tab, Sync sync, Mid mid) {
+    constexpr int G = LineShape<N>::G;
+    using L = SplitLine<N, G>;
+    fft_nat_to_spec_split<N, G, +1, STRIDE, G, TS>(v, o, t, h, sc, tab, sync);
+#pragma unroll
+    for (int r = 0; r < L::OUT; ++r) o[r] = mid(r, o[r]);
+    float2 w[L::IN];
+    if constexpr (L::Q == 1) {  // the pair's lanes exchange their outputs
+        sync();
+#pragma unroll
+        for (int r = 0; r < L::OUT; ++r) sc[(t * G + 2 * r + h) * STRIDE] = o[r];
+        sync();
+#pragma unroll
+        for (int r = 0; r < L::IN; ++r) w[r] = sc[(t * G + r) * STRIDE];
+    } else {
+#pragma unroll
+        for (int r = 0; r < L::OUT; ++r) w[r] = o[r];
+    }
+    fft_spec_to_nat_split<N, G, -1, STRIDE, G, TS>(w, o, t, h, sc, tab, sync);
+}
+
+// Row transforms of a line by LW consecutive lanes of a warp, between a row in memory (natural
+// frequency order) and the line buffer in shared memory (natural order). Lines of 16-point DFTs
+// (N >= 128) are split; 8-point ones save no more than the pairs' doubled loads cost (one 64 x 64
+// solve on the persistent grid 1105 us, split 1112; 256 x 256: 2.89 ms, split 2.63).
+template <int N, bool TS>
+struct RowLanes {
+    static constexpr int G = LineShape<N>::G, E = N / G;
+    static constexpr bool SPLIT = E >= 16;
+    static constexpr int LW = SPLIT ? 2 * G : G;
+    using L = SplitLine<N, G>;
+    int t, h;
+    float2 *line, *sc;  // sc: LineScratch<N, G>::SIZE
+    const float2 *tab;
+    __device__ RowLanes(int lane, float2 *l, float2 *s, const float2 *tb)
+        : t(lane % G), h(lane / G), line(l), sc(s), tab(tb) {}
+    // the transform of src (SIGN -1: to real space, +1: a first step's start) to dst
+    template <int SIGN>
+    __device__ __forceinline__ void to_spec(const float2 *src, float2 *dst) const {
+        float2 v[E];
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = src[t + G * j];
+        if constexpr (SPLIT) {
+            float2 o[L::OUT];
+            fft_nat_to_spec_split<N, G, SIGN, 1, G + 1, TS>(v, o, t, h, sc, tab, WarpSync());
+#pragma unroll
+            for (int r = 0; r < L::OUT; ++r) dst[L::spec(t, h, r)] = o[r];
+        } else {
+            fft_nat_to_spec<N, G, SIGN, false, 1, G + 1, TS>(v, t, sc, tab);
+#pragma unroll
+            for (int r = 0; r < E; ++r) dst[spec_index<N, G>(t, r)] = v[r];
+        }
+    }
+    // the backward transform of the line buffer to row F
+    __device__ __forceinline__ void start(float2 *F) const {
+        if constexpr (SPLIT) {
+            float2 v[L::IN], o[L::OUT];
+#pragma unroll
+            for (int r = 0; r < L::IN; ++r) v[r] = line[L::spec_in(t, h, r)];
+            fft_spec_to_nat_split<N, G, +1, 1, G + 1, TS>(v, o, t, h, sc, tab, WarpSync());
+#pragma unroll
+            for (int r = 0; r < L::OUT; ++r) F[L::nat(t, h, r)] = o[r];
+        } else {
+            float2 v[E];
+#pragma unroll
+            for (int r = 0; r < E; ++r) v[r] = line[spec_index<N, G>(t, r)];
+            fft_spec_to_nat<N, G, +1, false, 1, G + 1, TS>(v, t, sc, tab);
+#pragma unroll
+            for (int j = 0; j < E; ++j) F[t + G * j] = v[j];
+        }
+    }
+};
+
 // Propagator storage order. The column transforms (G = LineShape<N>::G threads per column,
 // E = N / G registers each) multiply register r of thread t by the propagator of spectral
 // row k = spec_index<N, G>(t, r) and column x. Registers r = 2j, 2j+1 of thread t form one
@@ -280,6 +500,26 @@ __device__ __forceinline__ void hprop_load(const float2 *__restrict__ H, int x, 
         const float4 q = __ldg(&SHG_AT(p, ((size_t)t * (E / 2) + j) * N + x, (size_t)N * N / 2, kChkPropagator));
         h[2 * j] = make_float2(q.x, q.y);
         h[2 * j + 1] = make_float2(q.z, q.w);
+    }
+}
+
+// The propagator values of split lane (t, h)'s outputs of column x.
+template <int N>
+__device__ __forceinline__ void split_hprop_load(const float2 *__restrict__ H, int x, int t, int h,
+                                                 float2 (&o)[N / LineShape<N>::G / 2]) {
+    constexpr int G = LineShape<N>::G, E = N / G;
+    if constexpr (E == G) {  // register 2 r + h: half h of word r
+#pragma unroll
+        for (int r = 0; r < E / 2; ++r)
+            o[r] = __ldg(&SHG_AT(H, (((size_t)t * (E / 2) + r) * N + x) * 2 + h, (size_t)N * N, kChkPropagator));
+    } else {  // registers h G + r: words h G / 2 + r / 2
+        const float4 *p = reinterpret_cast<const float4 *>(H);
+#pragma unroll
+        for (int r = 0; r < G / 2; ++r) {
+            const float4 q = __ldg(&SHG_AT(p, ((size_t)t * (E / 2) + h * (G / 2) + r) * N + x, (size_t)N * N / 2, kChkPropagator));
+            o[2 * r] = make_float2(q.x, q.y);
+            o[2 * r + 1] = make_float2(q.z, q.w);
+        }
     }
 }
 

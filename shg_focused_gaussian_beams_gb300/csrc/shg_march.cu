@@ -146,7 +146,7 @@ struct PtRowShape {
     static constexpr int LPB = (512 / N < N) ? 512 / N : N;
     static constexpr int TPB = LPB * N;
     static constexpr int BPI = N / LPB;
-    static constexpr int FT = LPB * G;  // transform threads per field
+    static constexpr int LW = RowLanes<N, false>::LW, FT = LPB * LW;  // transform lanes per field
     static_assert(FT % 32 == 0 && 2 * FT <= TPB && N % LPB == 0, "transform threads fill whole warps");
 };
 
@@ -158,16 +158,15 @@ template <int N, bool TS = false>
 __device__ __forceinline__ void rows_pt_body(const InstDesc &d, int line0, int s, float2 *scratch, float2 *lines0,
                                              float2 *lines1, const float2 *tab) {
     using Sh = PtRowShape<N>;
-    constexpr int G = Sh::G, E = N / G, LPB = Sh::LPB, FT = Sh::FT;
+    constexpr int G = Sh::G, LW = Sh::LW, LPB = Sh::LPB, FT = Sh::FT;
     constexpr int SC = LineScratch<N, G>::SIZE;
     const int tid = threadIdx.x;
     // transform role
     const bool xf = tid < 2 * FT;
-    const int f = tid / FT, fl = (tid % FT) / G, t = tid % G;
-    float2 *const F = f == 0 ? d.P : d.S;
+    const int f = tid / FT, fl = (tid % FT) / LW;
     float2 *const fline = ((f & 1) ? lines1 : lines0) + fl * N;
-    float2 *const fsc = scratch + (size_t)((f & 1) * LPB + fl) * SC;
-    const size_t fbase = (size_t)(line0 + fl) * N;
+    float2 *const F = (f == 0 ? d.P : d.S) + (size_t)(line0 + fl) * N;
+    const RowLanes<N, TS> xr(tid % LW, fline, scratch + (size_t)((f & 1) * LPB + fl) * SC, tab);
     // point role
     const int l = tid / N, x = tid % N;
     const size_t i2 = (size_t)(line0 + l) * N + x;
@@ -182,25 +181,11 @@ __device__ __forceinline__ void rows_pt_body(const InstDesc &d, int line0, int s
         *pP = vp;
         *pS = vs;
         __syncthreads();
-        if (xf) {
-            float2 v[E];
-#pragma unroll
-            for (int j = 0; j < E; ++j) v[j] = fline[t + G * j];
-            fft_nat_to_spec<N, G, +1, false, 1, G + 1, TS>(v, t, fsc, tab);
-#pragma unroll
-            for (int r = 0; r < E; ++r) F[fbase + spec_index<N, G>(t, r)] = v[r];
-        }
+        if (xf) xr.template to_spec<+1>(fline, F);
         return;
     }
     const float4 turn = d.stepc[s];  // before the transform, which hides its latency (s <= nsteps < nz)
-    if (xf) {
-        float2 v[E];
-#pragma unroll
-        for (int j = 0; j < E; ++j) v[j] = F[fbase + t + G * j];
-        fft_nat_to_spec<N, G, -1, false, 1, G + 1, TS>(v, t, fsc, tab);
-#pragma unroll
-        for (int r = 0; r < E; ++r) fline[spec_index<N, G>(t, r)] = v[r];
-    }
+    if (xf) xr.template to_spec<-1>(F, fline);
     __syncthreads();
     float2 vp = *pP, vs = *pS;
     rk4_march(vp, vs, d);
@@ -224,14 +209,7 @@ __device__ __forceinline__ void rows_pt_body(const InstDesc &d, int line0, int s
     *pP = vp;
     *pS = vs;
     __syncthreads();
-    if (xf) {
-        float2 v[E];
-#pragma unroll
-        for (int r = 0; r < E; ++r) v[r] = fline[spec_index<N, G>(t, r)];
-        fft_spec_to_nat<N, G, +1, false, 1, G + 1, TS>(v, t, fsc, tab);
-#pragma unroll
-        for (int j = 0; j < E; ++j) F[fbase + t + G * j] = v[j];
-    }
+    if (xf) xr.start(F);
 }
 
 template <int N>
@@ -262,19 +240,19 @@ __global__ void __launch_bounds__(TC * LineShape<N>::G) k_cols(const InstDesc *_
 // in one launch, separated by grid-wide barriers instead of kernel boundaries. A lone solve
 // otherwise pays two dependent launches per z-step.
 
-// Grid barrier, CoopShape and cols_body_h: shg_coop.cuh.
+// Grid barrier, CoopShape and CoopColumn: shg_coop.cuh.
 static_assert(CoopShape<64>::TPB == PtRowShape<64>::TPB && CoopShape<256>::ROW_UNITS == PtRowShape<256>::BPI &&
                   CoopShape<16>::TPB == PtRowShape<16>::TPB,
               "the persistent grid's row units are the row pass's blocks");
 
 // Grid of B blocks of TPB threads; block b runs row units b, b + B, ... and column groups
-// b + B w (warp w < col_warps), whose propagator values stay in registers for the whole run.
-// Dynamic shared memory: col_warps scratch regions of TC * N float2. bar: zeroed arrival
+// b + B w (warp w < col_groups), whose propagator values stay in registers for the whole run.
+// Dynamic shared memory: col_groups scratch regions of TC * N float2. bar: zeroed arrival
 // counter; err: zeroed error word of the run.
 template <int N>
 __global__ void __launch_bounds__(CoopShape<N>::TPB) k_march_coop(const InstDesc *__restrict__ inst,
                                                                  const int *__restrict__ list, unsigned *bar,
-                                                                 int *err, int col_warps) {
+                                                                 int *err, int col_groups) {
     using Sh = PtRowShape<N>;
     using C = CoopShape<N>;
     constexpr int G = Sh::G;
@@ -290,13 +268,10 @@ __global__ void __launch_bounds__(CoopShape<N>::TPB) k_march_coop(const InstDesc
         for (int i = threadIdx.x; i < N; i += blockDim.x) tws[i] = src[i];
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int K = d.nsteps;
-    const int u = blockIdx.x + gridDim.x * warp;
-    const bool colw = warp < col_warps && u < C::COL_UNITS;
-    const int f = u / (N / C::TC), x = (u % (N / C::TC)) * C::TC + lane % C::TC, t = lane / C::TC;
-    float2 h[C::E];
-    if (colw) hprop_load<N>(f == 0 ? d.Hp : d.Hs, x, t, h);
+    const CoopColumn<N> col(blockIdx.x, gridDim.x, col_groups);
+    float2 h[C::OUT];
+    if (col.active) col.load(d, h);
     unsigned target = 0;
     for (int s = 0; s <= K; ++s) {
         for (int r = blockIdx.x; r < C::ROW_UNITS; r += gridDim.x) {
@@ -306,7 +281,7 @@ __global__ void __launch_bounds__(CoopShape<N>::TPB) k_march_coop(const InstDesc
         if (s == K) break;
         target += gridDim.x;
         if (!grid_barrier(bar, target, err)) return;
-        if (colw) cols_body_h<N, C::TC>(d, x, f, t, cscr + (size_t)warp * C::TC * N + lane % C::TC, h, tws);
+        if (col.active) col.run(d, cscr, h, tws);
         target += gridDim.x;
         if (!grid_barrier(bar, target, err)) return;
     }
@@ -316,7 +291,7 @@ template <int N>
 static cudaError_t launch_coop_t(const InstDesc *inst, const int *list, unsigned *bar, int *err, cudaStream_t st,
                                  int *blocks_out) {
     using C = CoopShape<N>;
-    constexpr int warps = C::TPB / 32;
+    constexpr int groups = C::TPB / (32 * C::GW);  // column groups that a block can hold
     auto k = k_march_coop<N>;
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e;
@@ -324,19 +299,19 @@ static cudaError_t launch_coop_t(const InstDesc *inst, const int *list, unsigned
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     // one column group per block where that many blocks fit co-resident (the column pass
     // then spreads over the most SMs), else the fewest blocks that hold every row unit
-    int blocks = 0, col_warps = 0;
+    int blocks = 0, col_groups = 0;
     size_t smem = 0;
     for (int pass = 0; pass < 2 && !blocks; ++pass) {
         int b = C::ROW_UNITS;
         if (pass == 0 && C::COL_UNITS > b) b = C::COL_UNITS;
-        if ((C::COL_UNITS + warps - 1) / warps > b) b = (C::COL_UNITS + warps - 1) / warps;
+        if ((C::COL_UNITS + groups - 1) / groups > b) b = (C::COL_UNITS + groups - 1) / groups;
         const int cw = (C::COL_UNITS + b - 1) / b;
         const size_t sm = (size_t)cw * C::TC * N * sizeof(float2);
         if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
         if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, C::TPB, sm)) != cudaSuccess) return e;
         if (per_sm * sms >= b) {
             blocks = b;
-            col_warps = cw;
+            col_groups = cw;
             smem = sm;
         }
     }
@@ -353,7 +328,7 @@ static cudaError_t launch_coop_t(const InstDesc *inst, const int *list, unsigned
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, inst, list, bar, err, col_warps);
+    return cudaLaunchKernelEx(&cfg, k, inst, list, bar, err, col_groups);
 }
 
 cudaError_t launch_coop(int n, const InstDesc *inst, const int *list, unsigned *bar, int *err, cudaStream_t st,

@@ -438,7 +438,7 @@ struct ThRowShape {
     static constexpr int TPB = LPB * N;
     static constexpr int BPI = N / LPB;
     static_assert(LPB >= 1 && N % LPB == 0, "whole lines per block");
-    static constexpr int FFT_THREADS = LPB * G;  // per field
+    static constexpr int LW = RowLanes<N, false>::LW, FFT_THREADS = LPB * LW;  // per field (split lanes)
     static_assert(FFT_THREADS % 32 == 0 && 2 * FFT_THREADS <= TPB, "transform threads fill whole warps");
 };
 
@@ -460,20 +460,19 @@ __device__ __forceinline__ void rows_th_body(const InstDesc &d, const ThermDesc 
                                              float2 *scratch, float2 (*lines)[ThRowShape<N>::LPB * N],
                                              const float2 *tab, ThPoint &pt) {
     using Sh = ThRowShape<N>;
-    constexpr int G = Sh::G, E = N / G, LPB = Sh::LPB, FT = Sh::FFT_THREADS;
+    constexpr int G = Sh::G, LW = Sh::LW, LPB = Sh::LPB, FT = Sh::FFT_THREADS;
     constexpr int SC = LineScratch<N, G>::SIZE;
     // stages 0..nz: the THERMAL march runs one stage past the last slice (heat source of slice nz-1)
     if (!SHG_REQUIRE(d.n == N && s >= 0 && s <= th.nz && line0 >= 0 && line0 + LPB <= N, kChkThermalRows, s))
         return;  // block-uniform
     const size_t nxy = (size_t)N * N;
     const int tid = threadIdx.x;
-    // transform role: field f, line fl, thread t of the line
+    // transform role: field f, line fl
     const bool xf = tid < 2 * FT;
-    const int f = tid / FT, fl = (tid % FT) / G, t = tid % G;
-    float2 *const F = f == 0 ? d.P : d.S;
+    const int f = tid / FT, fl = (tid % FT) / LW;
     float2 *const fline = lines[f & 1] + fl * N;
-    float2 *const fsc = scratch + (size_t)((f & 1) * LPB + fl) * SC;
-    const size_t fbase = (size_t)(line0 + fl) * N;
+    float2 *const F = (f == 0 ? d.P : d.S) + (size_t)(line0 + fl) * N;
+    const RowLanes<N, KEEP> xr(tid % LW, fline, scratch + (size_t)((f & 1) * LPB + fl) * SC, tab);
     // point role: line l, column x
     const int l = tid / N, x = tid % N;
     const size_t i2 = (size_t)(line0 + l) * N + x;
@@ -491,28 +490,14 @@ __device__ __forceinline__ void rows_th_body(const InstDesc &d, const ThermDesc 
         *pP = vp;
         *pS = vs;
         __syncthreads();
-        if (xf) {
-            float2 v[E];
-#pragma unroll
-            for (int j = 0; j < E; ++j) v[j] = fline[t + G * j];
-            fft_nat_to_spec<N, G, +1, false, 1, G + 1, KEEP>(v, t, fsc, tab);
-#pragma unroll
-            for (int r = 0; r < E; ++r) F[fbase + spec_index<N, G>(t, r)] = v[r];
-        }
+        if (xf) xr.template to_spec<+1>(fline, F);
         return;
     }
     // the next slice's values first: their latency overlaps the transform
     const size_t i3 = (size_t)(s - 1) * nxy + i2, i3n = (size_t)(s < th.nz ? s : s - 1) * nxy + i2;
     const float npn = th.NP[i3n], nsn = th.NS[i3n], dkn = th.DK[i3n];
     // forward transform of the rows into natural x order
-    if (xf) {
-        float2 v[E];
-#pragma unroll
-        for (int j = 0; j < E; ++j) v[j] = F[fbase + t + G * j];
-        fft_nat_to_spec<N, G, -1, false, 1, G + 1, KEEP>(v, t, fsc, tab);
-#pragma unroll
-        for (int r = 0; r < E; ++r) fline[spec_index<N, G>(t, r)] = v[r];
-    }
+    if (xf) xr.template to_spec<-1>(F, fline);
     if (!KEEP) {
         pt.np = th.NP[i3];
         pt.ns = th.NS[i3];
@@ -563,14 +548,7 @@ __device__ __forceinline__ void rows_th_body(const InstDesc &d, const ThermDesc 
     if (s == th.nz) return;
     __syncthreads();
     // backward transform along x back to the column pass's layout
-    if (xf) {
-        float2 v[E];
-#pragma unroll
-        for (int r = 0; r < E; ++r) v[r] = fline[spec_index<N, G>(t, r)];
-        fft_spec_to_nat<N, G, +1, false, 1, G + 1, KEEP>(v, t, fsc, tab);
-#pragma unroll
-        for (int j = 0; j < E; ++j) F[fbase + t + G * j] = v[j];
-    }
+    if (xf) xr.start(F);
 }
 
 template <int N>
@@ -583,16 +561,16 @@ __global__ void __launch_bounds__(ThRowShape<N>::TPB) k_rows_th(const InstDesc *
 }
 
 // Persistent THERMAL march of one solve on a cooperative grid (stages 0..nz): the row pass
-// above and the plain column pass (cols_body_h, the same diffraction as k_cols) separated by
+// above and the plain column pass (CoopColumn, the same diffraction as k_cols) separated by
 // bounded grid-wide barriers instead of kernel boundaries. The grid has at least one block per
 // row unit: block b runs row unit b, whose points' constants stay in registers from stage to
-// stage, and column groups b + B w (warp w < col_warps), whose propagator values stay there for
+// stage, and column groups b + B w (warp w < col_groups), whose propagator values stay there for
 // the whole run. bar: zeroed arrival counter; err: the solve's error word, or-ed
 // with 2 when a barrier wait gave up.
 template <int N>
 __global__ void __launch_bounds__(ThRowShape<N>::TPB) k_march_coop_th(const InstDesc *__restrict__ dd,
                                                                       const ThermDesc th, unsigned *bar, int *err,
-                                                                      int col_warps) {
+                                                                      int col_groups) {
     using Sh = ThRowShape<N>;
     using C = CoopShape<N>;
     static_assert(C::TPB == Sh::TPB && C::ROW_UNITS == Sh::BPI, "row units are the row pass's blocks");
@@ -608,12 +586,9 @@ __global__ void __launch_bounds__(ThRowShape<N>::TPB) k_march_coop_th(const Inst
         for (int i = threadIdx.x; i < N; i += blockDim.x) tws[i] = src[i];
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int u = blockIdx.x + gridDim.x * warp;
-    const bool colw = warp < col_warps && u < C::COL_UNITS;
-    const int f = u / (N / C::TC), x = (u % (N / C::TC)) * C::TC + lane % C::TC, t = lane / C::TC;
-    float2 h[C::E];
-    if (colw) hprop_load<N>(f == 0 ? d.Hp : d.Hs, x, t, h);
+    const CoopColumn<N> col(blockIdx.x, gridDim.x, col_groups);
+    float2 h[C::OUT];
+    if (col.active) col.load(d, h);
     ThPoint pt;
     unsigned target = 0;
     for (int s = 0; s <= th.nz; ++s) {
@@ -622,7 +597,7 @@ __global__ void __launch_bounds__(ThRowShape<N>::TPB) k_march_coop_th(const Inst
         if (s == th.nz) break;
         target += gridDim.x;
         if (!grid_barrier(bar, target, err, 2)) return;
-        if (colw) cols_body_h<N, C::TC>(d, x, f, t, cscr + (size_t)warp * C::TC * N + lane % C::TC, h, tws);
+        if (col.active) col.run(d, cscr, h, tws);
         target += gridDim.x;
         if (!grid_barrier(bar, target, err, 2)) return;
     }
@@ -722,7 +697,7 @@ static cudaError_t launch_rows_th_t(const InstDesc *d, const ThermDesc &th, int 
 template <int N>
 static cudaError_t launch_coop_th_t(const InstDesc *d, const ThermDesc &th, unsigned *bar, int *err, cudaStream_t st) {
     using C = CoopShape<N>;
-    constexpr int warps = C::TPB / 32;
+    constexpr int groups = C::TPB / (32 * C::GW);  // column groups that a block can hold
     auto k = k_march_coop_th<N>;
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e;
@@ -730,19 +705,19 @@ static cudaError_t launch_coop_th_t(const InstDesc *d, const ThermDesc &th, unsi
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     // one column group per block where that many blocks fit co-resident, else the fewest
     // blocks that hold every row unit (as for the plain persistent grid)
-    int blocks = 0, col_warps = 0;
+    int blocks = 0, col_groups = 0;
     size_t smem = 0;
     for (int pass = 0; pass < 2 && !blocks; ++pass) {
         int b = C::ROW_UNITS;
         if (pass == 0 && C::COL_UNITS > b) b = C::COL_UNITS;
-        if ((C::COL_UNITS + warps - 1) / warps > b) b = (C::COL_UNITS + warps - 1) / warps;
+        if ((C::COL_UNITS + groups - 1) / groups > b) b = (C::COL_UNITS + groups - 1) / groups;
         const int cw = (C::COL_UNITS + b - 1) / b;
         const size_t sm = (size_t)cw * C::TC * N * sizeof(float2);
         if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
         if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, C::TPB, sm)) != cudaSuccess) return e;
         if (per_sm * sms >= b) {
             blocks = b;
-            col_warps = cw;
+            col_groups = cw;
             smem = sm;
         }
     }
@@ -758,7 +733,7 @@ static cudaError_t launch_coop_th_t(const InstDesc *d, const ThermDesc &th, unsi
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, d, th, bar, err, col_warps);
+    return cudaLaunchKernelEx(&cfg, k, d, th, bar, err, col_groups);
 }
 
 cudaError_t launch_coop_th(int n, const InstDesc *d, const ThermDesc &th, unsigned *bar, int *err, cudaStream_t st) {
