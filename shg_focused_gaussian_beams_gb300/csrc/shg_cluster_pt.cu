@@ -30,15 +30,10 @@ const float2 *twiddle_symbol_address_cluster_pt() {
 }
 SHG_CHECK_TU(cluster_pt)
 
-template <int N>
-struct CptCluster;
-template <> struct CptCluster<64> { static constexpr int CS = 8; };
-template <> struct CptCluster<128> { static constexpr int CS = 16; };
-template <> struct CptCluster<256> { static constexpr int CS = 16; };
-
-template <int N>
+// CS: CTAs per cluster (16: non-portable).
+template <int N, int CS_>
 struct CptShape {
-    static constexpr int CS = CptCluster<N>::CS;       // CTAs per cluster (16: non-portable)
+    static constexpr int CS = CS_;
     static constexpr int G = LineShape<N>::G, E = N / G;
     static constexpr int R = N / CS;                   // rows (and columns) per CTA
     static constexpr int TPB = 512;
@@ -68,10 +63,10 @@ __device__ __forceinline__ void cpt_block_add(double v, double *dst) {
 }
 
 // Grid: count clusters of CS CTAs, cluster c marching solve list[c].
-template <int N>
-__global__ void __launch_bounds__(CptShape<N>::TPB, 1)
+template <int N, int CS>
+__global__ void __launch_bounds__(CptShape<N, CS>::TPB, 1)
     k_march_cluster_pt(const InstDesc *__restrict__ inst, const int *__restrict__ list) {
-    using Sh = CptShape<N>;
+    using Sh = CptShape<N, CS>;
     constexpr int G = Sh::G, E = Sh::E, R = Sh::R, N2 = R * G, TC = Sh::TC, FIELD = Sh::FIELD;
     extern __shared__ float2 smem[];
     float2 *const sP = smem, *const sS = smem + FIELD, *const scr = smem + 2 * FIELD;
@@ -219,9 +214,9 @@ __global__ void __launch_bounds__(CptShape<N>::TPB, 1)
     // writes another's shared memory after that, so CTAs may exit independently.
 }
 
-template <int N>
+template <int N, int CS>
 static cudaLaunchConfig_t cpt_config(cudaLaunchAttribute *attr, cudaStream_t st) {
-    using Sh = CptShape<N>;
+    using Sh = CptShape<N, CS>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(Sh::TPB, 1, 1);
     cfg.dynamicSmemBytes = Sh::SMEM;
@@ -235,54 +230,62 @@ static cudaLaunchConfig_t cpt_config(cudaLaunchAttribute *attr, cudaStream_t st)
     return cfg;
 }
 
-template <int N>
+template <int N, int CS>
 static cudaError_t prepare_cpt_t(int *max_clusters) {
-    using Sh = CptShape<N>;
-    auto k = k_march_cluster_pt<N>;
+    using Sh = CptShape<N, CS>;
+    auto k = k_march_cluster_pt<N, CS>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM);
     if (e != cudaSuccess) return e;
     if (Sh::CS > 8 && (e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
         return e;
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = cpt_config<N>(attr, nullptr);
+    cudaLaunchConfig_t cfg = cpt_config<N, CS>(attr, nullptr);
     cfg.gridDim = dim3(Sh::CS, 1, 1);
     return cudaOccupancyMaxActiveClusters(max_clusters, k, &cfg);
 }
 
-template <int N>
+template <int N, int CS>
 static cudaError_t launch_cpt_t(const InstDesc *inst, const int *list, int count, cudaStream_t st) {
-    using Sh = CptShape<N>;
+    using Sh = CptShape<N, CS>;
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = cpt_config<N>(attr, st);
+    cudaLaunchConfig_t cfg = cpt_config<N, CS>(attr, st);
     cfg.gridDim = dim3((unsigned)count * Sh::CS, 1, 1);
-    return cudaLaunchKernelEx(&cfg, k_march_cluster_pt<N>, inst, list);
+    return cudaLaunchKernelEx(&cfg, k_march_cluster_pt<N, CS>, inst, list);
 }
 
-int cluster_pt_size(int n) {
+// Cluster sizes of a grid, largest first. A wave of CTAs (one per SM) holds fewer solves of a larger
+// cluster, which marches each faster. (Clusters of two and, for 128 x 128, of four lose to the resident
+// march, whose smaller CTAs share an SM: 38 solves of 64 x 64 x 200 1.51 against 1.46 ms, 18 of 128 x 128
+// 3.04 against 2.70.)
+int cluster_pt_sizes(int n, int *out) {
     switch (n) {
-        case 64: return CptShape<64>::CS;
-        case 128: return CptShape<128>::CS;
-        case 256: return CptShape<256>::CS;
+        case 64: out[0] = 8, out[1] = 4; return 2;
+        case 128: out[0] = 16, out[1] = 8; return 2;
+        case 256: out[0] = 16; return 1;
         default: return 0;
     }
 }
 
-cudaError_t prepare_cluster_pt(int n, int *max_clusters) {
+cudaError_t prepare_cluster_pt(int n, int cs, int *max_clusters) {
     *max_clusters = 0;
-    switch (n) {
-        case 64: return prepare_cpt_t<64>(max_clusters);
-        case 128: return prepare_cpt_t<128>(max_clusters);
-        case 256: return prepare_cpt_t<256>(max_clusters);
+    switch (n * 100 + cs) {
+        case 6408: return prepare_cpt_t<64, 8>(max_clusters);
+        case 6404: return prepare_cpt_t<64, 4>(max_clusters);
+        case 12816: return prepare_cpt_t<128, 16>(max_clusters);
+        case 12808: return prepare_cpt_t<128, 8>(max_clusters);
+        case 25616: return prepare_cpt_t<256, 16>(max_clusters);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t launch_cluster_pt(int n, const InstDesc *inst, const int *list, int count, cudaStream_t st) {
+cudaError_t launch_cluster_pt(int n, int cs, const InstDesc *inst, const int *list, int count, cudaStream_t st) {
     if (count < 1) return cudaErrorInvalidValue;
-    switch (n) {
-        case 64: return launch_cpt_t<64>(inst, list, count, st);
-        case 128: return launch_cpt_t<128>(inst, list, count, st);
-        case 256: return launch_cpt_t<256>(inst, list, count, st);
+    switch (n * 100 + cs) {
+        case 6408: return launch_cpt_t<64, 8>(inst, list, count, st);
+        case 6404: return launch_cpt_t<64, 4>(inst, list, count, st);
+        case 12816: return launch_cpt_t<128, 16>(inst, list, count, st);
+        case 12808: return launch_cpt_t<128, 8>(inst, list, count, st);
+        case 25616: return launch_cpt_t<256, 16>(inst, list, count, st);
         default: return cudaErrorInvalidValue;
     }
 }

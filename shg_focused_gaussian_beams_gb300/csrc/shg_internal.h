@@ -52,7 +52,7 @@ cudaError_t launch_check_selftest(long long value);
 struct ResidentVariant {
     int cs, minb, g;  // cluster size, CTAs per SM, threads per line (FFT split N = (N/g) x g);
                       // cs == 0: the persistent cooperative grid of one solve (launch_coop);
-                      // cs == -1: one cluster per solve, one thread per point in the
+                      // cs == -1: one cluster of g CTAs per solve, one thread per point in the
                       // pointwise phase (launch_cluster_pt); cs == -2: persistent groups of
                       // blocks (launch_group)
 };
@@ -75,12 +75,12 @@ cudaError_t launch_coop(int n, const InstDesc *inst, const int *list, unsigned *
 bool line_length_supported(int n);
 
 // shg_cluster_pt.cu: the march of each of `count` solves (list[0..count)) in one
-// thread-block cluster of cluster_pt_size(n) CTAs, both fields in the cluster's shared
+// thread-block cluster of cs CTAs (one of cluster_pt_sizes), both fields in the cluster's shared
 // memory (n in {64, 128, 256}). prepare_cluster_pt: once per device, outside any capture;
 // max_clusters receives how many clusters fit at once (0: none).
-int cluster_pt_size(int n);
-cudaError_t prepare_cluster_pt(int n, int *max_clusters);
-cudaError_t launch_cluster_pt(int n, const InstDesc *inst, const int *list, int count, cudaStream_t st);
+int cluster_pt_sizes(int n, int *out);  // up to 2
+cudaError_t prepare_cluster_pt(int n, int cs, int *max_clusters);
+cudaError_t launch_cluster_pt(int n, int cs, const InstDesc *inst, const int *list, int count, cudaStream_t st);
 // shg_group.cu: the march of `njobs` solves (list[0..njobs)) by persistent groups of blocks with
 // bounded barriers, one cooperative launch (n in {64, 128, 256}). words: kGroupWords zeroed words;
 // err: zeroed, set when a barrier wait gave up. inst == nullptr only counts the groups that fit
