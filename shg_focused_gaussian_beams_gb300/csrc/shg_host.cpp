@@ -311,11 +311,15 @@ class Batch {
         const size_t region = al(pts * sizeof(float2));
         const size_t step_off = 6 * region;
         const size_t acc_off = step_off + al(nz_total * sizeof(float4));
-        const size_t total = acc_off + al(4 * sizeof(double) * n);
+        const size_t total = acc_off + al(4 * sizeof(double) * n + sizeof(double));  // the error word behind the sums
         SHG_TRY_INT(device_fits(total, "batch"));
         SHG_CUDA(cudaMalloc(&pool_, total));
         pool_bytes_ = total;
         acc_ = reinterpret_cast<double *>(pool_ + acc_off);
+        if (cudaMallocHost(&h_tail_, (4 * (size_t)n + 1) * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            h_tail_ = nullptr;  // the sums are then read from the device
+        }
         desc_.resize(n);
         p_src_.assign(n, nullptr);
         s_src_.assign(n, nullptr);
@@ -505,6 +509,11 @@ class Batch {
             SHG_CUDA(cudaMemcpyAsync(d_desc_, desc_.data(), desc_.size() * sizeof(InstDesc), cudaMemcpyHostToDevice, st));
             desc_dirty_ = false;
         }
+        tail_ready_ = false;
+        // a run captured into the caller's graph may be replayed at any time: no copy stays current
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        SHG_CUDA(cudaStreamIsCapturing(st, &cs));
+        if (cs != cudaStreamCaptureStatusNone) captured_ = true;
         if (!use_graph) return enqueue(st);
         if (!graph_exec_) {
             // Capture on a private stream (the caller's may be the legacy default stream,
@@ -524,6 +533,17 @@ class Batch {
             SHG_CUDA(e);
         }
         SHG_CUDA(cudaGraphLaunch(graph_exec_, st));
+        return SHG_OK;
+    }
+
+    // Waits for the run enqueued on st, with its sums and error word copied to pinned memory on the way:
+    // read_tail then needs no copy of its own (a lone solve's run, fields and efficiency took four
+    // blocking ones of about 5 us each; 32 x 32 x 48 279 -> 262 us).
+    int wait_run(cudaStream_t st) {
+        if (h_tail_)
+            SHG_CUDA(cudaMemcpyAsync(h_tail_, acc_, (4 * desc_.size() + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
+        SHG_CUDA(cudaStreamSynchronize(st));
+        tail_ready_ = h_tail_ && !captured_;
         return SHG_OK;
     }
 
@@ -887,17 +907,32 @@ class Batch {
         return out;
     }
 
-    int copy_acc(std::vector<double> &acc) {
-        acc.resize(4 * desc_.size());
-        SHG_CUDA(cudaMemcpy(acc.data(), acc_, acc.size() * sizeof(double), cudaMemcpyDeviceToHost));
-        return check_run_errors();
+    // Sums and error word (set when a barrier wait of a persistent grid gave up) of the last run,
+    // read after the run has completed.
+    int read_tail(std::vector<double> &t) {
+        t.resize(4 * desc_.size() + 1);
+        const size_t bytes = t.size() * sizeof(double);
+        if (tail_ready_)
+            std::memcpy(t.data(), h_tail_, bytes);
+        else
+            SHG_CUDA(cudaMemcpy(t.data(), acc_, bytes, cudaMemcpyDeviceToHost));
+        return SHG_OK;
     }
 
-    // Error word of the last run (set when a grid-barrier wait of the persistent grid gave up);
-    // read after the run has completed.
+    int copy_acc(std::vector<double> &acc) {
+        SHG_TRY_INT(read_tail(acc));
+        return check_tail(acc);
+    }
+
     int check_run_errors() {
+        std::vector<double> t;
+        SHG_TRY_INT(read_tail(t));
+        return check_tail(t);
+    }
+
+    int check_tail(const std::vector<double> &t) {
         int flag = 0;
-        SHG_CUDA(cudaMemcpy(&flag, d_counters_ + 63, sizeof(int), cudaMemcpyDeviceToHost));
+        std::memcpy(&flag, &t.back(), sizeof(int));
         if (flag) {
             set_error("persistent grid: a grid-barrier wait gave up (run incomplete)");
             return SHG_ERR_CUDA;
@@ -1011,7 +1046,8 @@ class Batch {
     // one behind the other: one memset per run of them (one per solve cost 1 us each, 25 of 960 us of
     // 24 solves of 64 x 64 x 200).
     int enqueue_inputs(cudaStream_t st) {
-        SHG_CUDA(cudaMemsetAsync(acc_, 0, 4 * sizeof(double) * desc_.size(), st));
+        tail_ready_ = false;
+        SHG_CUDA(cudaMemsetAsync(acc_, 0, 4 * sizeof(double) * desc_.size() + sizeof(double), st));
         const int n = (int)desc_.size();
         for (int i = 0; i < n; ++i) {
             const size_t bytes = (size_t)desc_[i].n * desc_[i].n * sizeof(float2);
@@ -1064,18 +1100,18 @@ class Batch {
         const Class &k = classes_[ci];
         const int *list = d_lists_ + k.offset;
         if (k.resident && k.var.cs == 0) {
-            // the persistent cooperative grid of a lone solve: barrier words 40 + 2 ci, error word 63
+            // the persistent cooperative grid of a lone solve: barrier words 40 + 2 ci
             unsigned *bar = reinterpret_cast<unsigned *>(d_counters_ + 40 + 2 * ci);
             if (rec) SHG_TRY_INT(rec->begin("coop<" + std::to_string(k.n) + ">", 32.0 * k.pt_steps, st));
-            SHG_CUDA(launch_coop(k.n, d_desc_, list, bar, d_counters_ + 63, st));
+            SHG_CUDA(launch_coop(k.n, d_desc_, list, bar, err_word(), st));
             if (rec) SHG_TRY_INT(rec->end(st));
             return SHG_OK;
         }
         if (k.resident && k.var.cs == -2) {
-            // the persistent groups: words of grid 64, 128, 256 after the first 64, error word 63
+            // the persistent groups: words of grid 64, 128, 256 after the first 64
             unsigned *words = reinterpret_cast<unsigned *>(d_counters_ + 64) + (k.n == 64 ? 0 : k.n == 128 ? 1 : 2) * kGroupWords;
             if (rec) SHG_TRY_INT(rec->begin("group<" + std::to_string(k.n) + ">", 32.0 * k.pt_steps, st));
-            SHG_CUDA(launch_group(k.n, d_desc_, list, k.count, words, d_counters_ + 63, st));
+            SHG_CUDA(launch_group(k.n, d_desc_, list, k.count, words, err_word(), st));
             if (rec) SHG_TRY_INT(rec->end(st));
             return SHG_OK;
         }
@@ -1133,6 +1169,9 @@ class Batch {
         d_counters_ = nullptr;
         if (capture_stream_) cudaStreamDestroy(capture_stream_);
         capture_stream_ = nullptr;
+        if (h_tail_) cudaFreeHost(h_tail_);
+        h_tail_ = nullptr;
+        tail_ready_ = captured_ = false;
         if (pool_) cudaFree(pool_);
         if (d_desc_) cudaFree(d_desc_);
         if (d_lists_) cudaFree(d_lists_);
@@ -1150,14 +1189,19 @@ class Batch {
     std::vector<Class> classes_;
     char *pool_ = nullptr;
     size_t pool_bytes_ = 0;
-    double *acc_ = nullptr;
+    int *err_word() const { return reinterpret_cast<int *>(acc_ + 4 * desc_.size()); }
+
+    double *acc_ = nullptr;       // 4 per solve, then the run's error word
+    double *h_tail_ = nullptr;    // pinned copy of both
+    bool tail_ready_ = false;     // it holds the last run's
+    bool captured_ = false;       // a run was captured into a caller's graph
     InstDesc *d_desc_ = nullptr;
     int *d_lists_ = nullptr;
     int max_nn_ = 0, max_nz_ = 0;
     bool desc_dirty_ = true;
     cudaGraphExec_t graph_exec_ = nullptr;
     cudaStream_t capture_stream_ = nullptr;
-    // job counters, barrier and error words of a run: 64 words, then those of the persistent groups
+    // job counters and barrier words of a run: 64 words, then those of the persistent groups
     static constexpr size_t kCounterBytes = (64 + 3 * (size_t)kGroupWords) * sizeof(int);
     int *d_counters_ = nullptr;
     std::vector<std::pair<std::string, float>> mix_;  // concurrent-run trials of the autotuner
@@ -1444,7 +1488,7 @@ int shg_cwes(shg_handle *h, float temp) {
     h->sp.temp = temp;
     h->sp.tprop = temp;
     SHG_TRY(handle_run(h, h->stream));
-    SHG_CUDA(cudaStreamSynchronize(h->stream));
+    SHG_TRY(h->batch.wait_run(h->stream));
     if (!h->th) SHG_TRY(h->batch.check_run_errors());
     return SHG_OK;
 }
@@ -1515,7 +1559,7 @@ int shg_run(shg_handle *h, float power, float waist, float focalpoint, float tem
         SHG_CUDA(cudaMalloc(&h->slices, (size_t)h->cfg.nz * 2 * h->n * h->n * sizeof(float2)));
     h->batch.set_slices(0, per_slice ? h->slices : nullptr);
     SHG_TRY(handle_run(h, h->stream));
-    SHG_CUDA(cudaStreamSynchronize(h->stream));
+    SHG_TRY(h->batch.wait_run(h->stream));
     if (!h->th) SHG_TRY(h->batch.check_run_errors());
     if (!h->out_dir.empty()) SHG_TRY(write_outputs(h, save_only_last, false));
     return SHG_OK;
@@ -1789,7 +1833,7 @@ int shg_batch_run(shg_batch *b, double *eta, float *sh_out_all) {
     if (sh_out_all)
         SHG_CUDA(cudaMemcpyAsync(sh_out_all, b->batch.sout_all(), b->batch.total_points() * sizeof(float2),
                                  cudaMemcpyDeviceToHost, b->stream));
-    SHG_CUDA(cudaStreamSynchronize(b->stream));
+    SHG_TRY(b->batch.wait_run(b->stream));
     if (eta)
         SHG_TRY(shg_batch_results(b, eta));
     else
