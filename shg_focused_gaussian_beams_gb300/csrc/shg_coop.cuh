@@ -29,7 +29,9 @@ __device__ __forceinline__ void red_release_gpu(unsigned *p, unsigned v) {
 // block barrier made its own, before the arrival) and polls with acquire loads (ordering
 // the other blocks' writes before this block's later loads). No reset step: a waiter reads
 // one word. Every wait is bounded: on timeout `code` is or-ed into *err and false is
-// returned (the caller leaves the kernel), and a wait also ends once *err is non-zero.
+// returned (the caller leaves the kernel), and a wait also ends once *err is non-zero (looked at on
+// every 32nd poll: read on each, it doubled the interval between polls; one 128 x 128 x 200 march
+// 1.19 -> 1.13 ms without).
 __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, int *err, int code = 1) {
     __shared__ int ok;
     __syncthreads();
@@ -37,12 +39,13 @@ __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, i
         red_release_gpu(count, 1u);
         int good = 1;
         for (long long it = 0; ld_acquire_gpu(count) < target; ++it) {
+            if ((it & 31) != 31) continue;
             if (it >= kGridWaitLimit || *(volatile int *)err) {
                 atomicOr(err, code);
                 good = 0;
                 break;
             }
-            if (it >= 64) __nanosleep(32);
+            if (it >= 127) __nanosleep(1000);
         }
         ok = good;
     }
