@@ -38,9 +38,7 @@ SHG_CHECK_TU(adjoint)
 // A and Fst hold the fields back to back (solve-major), acc[blockIdx.y] receives the sums.
 // TC columns per block: 16 when several solves fill the GPU, 4 for one to three solves
 // (N >= 64, so that a block holds whole warps).
-// CHAINED: launched by launch_dependent (the batched THERMAL pass; of the plain adjoint, whose replay
-// branch runs at another priority, programmatic launches cost 2 %).
-template <int N, int MODE, int TC, bool CHAINED>
+template <int N, int MODE, int TC>
 __global__ void __launch_bounds__(TC * LineShape<N>::G) k_colpass(float2 *A0, float2 *Fst0,
                                                              const InstDesc *__restrict__ dd, double *acc0) {
     constexpr int G = LineShape<N>::G, E = N / G;
@@ -66,7 +64,7 @@ __global__ void __launch_bounds__(TC * LineShape<N>::G) k_colpass(float2 *A0, fl
 #pragma unroll
         for (int r = 0; r < E; ++r) fv[r] = Fst[(size_t)spec_index<N, G>(t, r) * N + x];
     }
-    if constexpr (CHAINED) grid_dependency_wait();
+    grid_dependency_wait();
     float2 v[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) v[j] = A[(size_t)(t + G * j) * N + x];
@@ -122,6 +120,7 @@ __global__ void __launch_bounds__(AdjRowShape<N>::TPB)
     const float2 *__restrict__ tab = g_twiddle + N;
     const size_t nn = (size_t)N * N;
     Cx cx(lines, scratch);
+    grid_dependency_wait();
     float2 p, q;
     if (finish) {
         cx.finish(A, tab);
@@ -180,7 +179,8 @@ __global__ void __launch_bounds__(AdjRowShape<N>::TPB)
     const float hp = d.hp, t0 = d.tpa0, t1 = d.tpa1, w6 = d.dz6;
     Cx cx(lines, scratch);
     float a1[5] = {0, 0, 0, 0, 0}, a2[5] = {0, 0, 0, 0, 0};  // this point's sums, FP64 across points
-    // the stored states of this point first: their latency overlaps the transform
+    // the stored states of this point first (written before the pass that precedes this one
+    // began): their latency overlaps its end and the transform
     float2 xp = make_float2(0.f, 0.f), xs = xp, wp = xp, ws = xp;
     if (finish) {
         xp = Xn[cx.i2];
@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(AdjRowShape<N>::TPB)
         wp = Wn[cx.i2];
         ws = Wn[nn + cx.i2];
     }
+    grid_dependency_wait();
     float2 cp, cs;
     if (finish) {
         cx.finish(C, tab);
@@ -321,36 +322,30 @@ static int grid_for(int nn) {
 
 template <int N, int TC>
 static cudaError_t launch_colpass_tc(int mode, float2 *A, float2 *F, const InstDesc *d, double *acc, int solves,
-                                     bool chained, cudaStream_t st) {
+                                     cudaStream_t st) {
     constexpr int G = LineShape<N>::G;
     const dim3 grid(N / TC, 2 * solves);
-    if (chained)
-        return launch_dependent(mode == 0 ? k_colpass<N, 0, TC, true> : k_colpass<N, 2, TC, true>, grid, TC * G, st, A, F,
-                                d, acc);
-    if (mode == 0)
-        k_colpass<N, 0, TC, false><<<grid, TC * G, 0, st>>>(A, F, d, acc);
-    else
-        k_colpass<N, 1, TC, false><<<grid, TC * G, 0, st>>>(A, F, d, acc);
-    return cudaGetLastError();
+    auto k = mode == 0 ? k_colpass<N, 0, TC> : mode == 1 ? k_colpass<N, 1, TC> : k_colpass<N, 2, TC>;
+    return launch_dependent(k, grid, TC * G, st, A, F, d, acc);
 }
 
 template <int N>
 static cudaError_t launch_colpass_t(int mode, float2 *A, float2 *F, const InstDesc *d, double *acc, int solves,
-                                    bool chained, cudaStream_t st) {
+                                    cudaStream_t st) {
     // narrow tiles only where a block still fills a warp (the sums use full-warp shuffles)
-    if (solves >= 4 || 4 * LineShape<N>::G < 32) return launch_colpass_tc<N, 16>(mode, A, F, d, acc, solves, chained, st);
-    return launch_colpass_tc<N, 4>(mode, A, F, d, acc, solves, chained, st);
+    if (solves >= 4 || 4 * LineShape<N>::G < 32) return launch_colpass_tc<N, 16>(mode, A, F, d, acc, solves, st);
+    return launch_colpass_tc<N, 4>(mode, A, F, d, acc, solves, st);
 }
 
 cudaError_t launch_colpass(int n, int mode, float2 *A, float2 *F, const InstDesc *d, double *acc, cudaStream_t st,
-                           int solves, bool chained) {
-    if (solves < 1 || solves > 32767 || mode == (chained ? 1 : 2)) return cudaErrorInvalidValue;
+                           int solves) {
+    if (solves < 1 || solves > 32767) return cudaErrorInvalidValue;
     switch (n) {
-        case 16: return launch_colpass_t<16>(mode, A, F, d, acc, solves, chained, st);
-        case 32: return launch_colpass_t<32>(mode, A, F, d, acc, solves, chained, st);
-        case 64: return launch_colpass_t<64>(mode, A, F, d, acc, solves, chained, st);
-        case 128: return launch_colpass_t<128>(mode, A, F, d, acc, solves, chained, st);
-        case 256: return launch_colpass_t<256>(mode, A, F, d, acc, solves, chained, st);
+        case 16: return launch_colpass_t<16>(mode, A, F, d, acc, solves, st);
+        case 32: return launch_colpass_t<32>(mode, A, F, d, acc, solves, st);
+        case 64: return launch_colpass_t<64>(mode, A, F, d, acc, solves, st);
+        case 128: return launch_colpass_t<128>(mode, A, F, d, acc, solves, st);
+        case 256: return launch_colpass_t<256>(mode, A, F, d, acc, solves, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -359,18 +354,16 @@ template <int N>
 static cudaError_t launch_adj_rows_fwd_t(const InstDesc *d, float2 *A, int s, int finish, int start, const float2 *inP,
                                          const float2 *inS, float2 *w_out, float2 *x_out, float2 *ck_out,
                                          float2 *final_out, cudaStream_t st) {
-    k_adj_rows_fwd<N><<<AdjRowShape<N>::BPI, AdjRowShape<N>::TPB, 0, st>>>(d, A, s, finish, start, inP, inS, w_out,
-                                                                            x_out, ck_out, final_out);
-    return cudaGetLastError();
+    return launch_dependent(k_adj_rows_fwd<N>, dim3(AdjRowShape<N>::BPI), AdjRowShape<N>::TPB, st, d, A, s, finish,
+                            start, inP, inS, w_out, x_out, ck_out, final_out);
 }
 
 template <int N>
 static cudaError_t launch_adj_rows_bwd_t(const InstDesc *d, float2 *C, int s, int finish, int start,
                                          const float2 *Xn, const float2 *Wn, double *acc_fin, double *acc_start,
                                          cudaStream_t st) {
-    k_adj_rows_bwd<N><<<AdjRowShape<N>::BPI, AdjRowShape<N>::TPB, 0, st>>>(d, C, s, finish, start, Xn, Wn, acc_fin,
-                                                                            acc_start);
-    return cudaGetLastError();
+    return launch_dependent(k_adj_rows_bwd<N>, dim3(AdjRowShape<N>::BPI), AdjRowShape<N>::TPB, st, d, C, s, finish,
+                            start, Xn, Wn, acc_fin, acc_start);
 }
 
 cudaError_t launch_adj_rows_fwd(int n, const InstDesc *d, float2 *A, int s, int finish, int start, const float2 *inP,

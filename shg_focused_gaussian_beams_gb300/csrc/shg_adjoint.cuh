@@ -7,25 +7,6 @@
 
 namespace shg {
 
-// The passes of a z step form a chain, each reading what the one before it wrote. Launched with
-// programmatic serialisation, a pass starts while its predecessor drains, fetches what no pass
-// writes (propagator, coefficients) and waits here for the predecessor's results.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <class... P, class... A>
-inline cudaError_t launch_dependent(void (*k)(P...), dim3 grid, int threads, cudaStream_t st, A... a) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, P(a)...);
-}
-
 // Adds the block's k partial sums (k <= 6) to dst[0..k) with one FP64 atomic each.
 __device__ __forceinline__ void block_sum_doubles(double *v, int k, double *dst) {
     __shared__ double red[32][6];

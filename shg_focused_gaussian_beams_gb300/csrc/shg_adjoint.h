@@ -10,10 +10,9 @@ namespace shg {
 
 // Column pass of the diffraction over `solves` solves (d[solves], fields solve-major):
 // mode 0 forward (spectra into F when F != nullptr), 1 adjoint with the propagator
-// sums into acc[2*solves], 2 adjoint without sums. chained: launched with programmatic
-// serialisation (launch_dependent); mode 1 unchained, mode 2 chained only.
+// sums into acc[2*solves], 2 adjoint without sums.
 cudaError_t launch_colpass(int n, int mode, float2 *A, float2 *F, const InstDesc *d, double *acc, cudaStream_t st,
-                           int solves = 1, bool chained = false);
+                           int solves = 1);
 // Fused row passes of one solve (one row launch per step boundary, see shg_adjoint.cu):
 // forward at boundary s (finish the diffraction of step s-1 and RK4 into X_s, or take X_s
 // from inP / inS; store W_{s-1}, X_s where asked; RK4 and start step s, or store X_K);

@@ -219,7 +219,7 @@ int ThermalGradBatch::enqueue(bool grad, int L, int nseg, bool store_all, cudaSt
     ++nl;
     // between two row passes: the y transforms and the propagator
     auto columns = [&](float2 *A, int mode, cudaStream_t q) -> int {
-        TG_CUDA(launch_colpass(n, mode, A, nullptr, d_desc_, nullptr, q, B, true));
+        TG_CUDA(launch_colpass(n, mode, A, nullptr, d_desc_, nullptr, q, B));
         ++nl;
         return SHG_OK;
     };

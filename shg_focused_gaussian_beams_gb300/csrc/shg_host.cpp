@@ -1136,7 +1136,7 @@ class Batch {
             if (rec) SHG_TRY_INT(rec->end(st));
             if (nc > 0) {
                 if (rec) SHG_TRY_INT(rec->begin(cn, 48.0 * nn * nc, st));
-                SHG_CUDA(launch_cols(k.n, d_desc_, list, nc, st));
+                SHG_CUDA(launch_cols(k.n, d_desc_, list, nc, s, st));
                 if (rec) SHG_TRY_INT(rec->end(st));
             }
         }

@@ -66,7 +66,7 @@ cudaError_t launch_resident(int n, ResidentVariant v, const InstDesc *inst, cons
 // frame: stepc as the plain march reads it, else as the adjoint does (InstDesc).
 cudaError_t launch_setup(const InstDesc *inst, int n_inst, int max_nn, int max_nz, bool frame, cudaStream_t st);
 cudaError_t launch_rows(int n, const InstDesc *inst, const int *list, int count, int s, cudaStream_t st);
-cudaError_t launch_cols(int n, const InstDesc *inst, const int *list, int count, cudaStream_t st);
+cudaError_t launch_cols(int n, const InstDesc *inst, const int *list, int count, int s, cudaStream_t st);
 // The whole march of one solve (list[0]) as one cooperative launch with bounded grid
 // barriers (bar: two zeroed words; err: zeroed, set to 1 when a barrier wait gave up).
 // inst == nullptr only checks that the grid fits co-resident; blocks receives its size.

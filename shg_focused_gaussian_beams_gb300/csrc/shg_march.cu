@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(PtRowShape<N>::TPB) k_rows_pt(const InstDesc *
     using Sh = PtRowShape<N>;
     __shared__ float2 scratch[2 * Sh::LPB * LineScratch<N, Sh::G>::SIZE];
     __shared__ float2 lines[2][Sh::LPB * N];  // [field][line * N + x], natural x order
+    grid_dependency_wait();
     const InstDesc &d = inst[list[blockIdx.x / Sh::BPI]];
     if (!check_solve<N>(d, s)) return;  // whole block
     rows_pt_body<N>(d, (blockIdx.x % Sh::BPI) * Sh::LPB, s, scratch, lines[0], lines[1], g_twiddle + N);
@@ -225,13 +226,15 @@ __global__ void __launch_bounds__(PtRowShape<N>::TPB) k_rows_pt(const InstDesc *
 // Column pass. Block = TC columns x G threads (lane = column + TC * t) so that every
 // load and store is a run of TC consecutive complex values; blockIdx.y = field (pump, SH).
 template <int N, int TC>
-__global__ void __launch_bounds__(TC * LineShape<N>::G) k_cols(const InstDesc *__restrict__ inst, const int *__restrict__ list) {
+__global__ void __launch_bounds__(TC * LineShape<N>::G) k_cols(const InstDesc *__restrict__ inst, const int *__restrict__ list, int s) {
     constexpr int G = LineShape<N>::G, E = N / G, BPI = N / TC;
     __shared__ float2 scratch[TC * E * G];
     const int c = threadIdx.x % TC;
     const InstDesc &d = inst[list[blockIdx.x / BPI]];
     if (!SHG_REQUIRE(d.n == N, kChkDescriptor, d.n)) return;
-    cols_body<N, TC, true>(d, (blockIdx.x % BPI) * TC + c, blockIdx.y, threadIdx.x / TC, scratch + c, g_twiddle + N);
+    if (s == 0) grid_dependency_wait();  // the set-up's propagators
+    cols_body<N, TC, true>(d, (blockIdx.x % BPI) * TC + c, blockIdx.y, threadIdx.x / TC, scratch + c, g_twiddle + N,
+                           [] { grid_dependency_wait(); });
 }
 
 // ---------------------------------------------------------------------------------------
@@ -412,20 +415,20 @@ static cudaError_t launch_rows_t(const InstDesc *inst, const int *list, int coun
     if (count >= 4)
         k_rows<N><<<count * RowShape<N>::BPI, RowShape<N>::TPB, 0, st>>>(inst, list, s);
     else
-        k_rows_pt<N><<<count * PtRowShape<N>::BPI, PtRowShape<N>::TPB, 0, st>>>(inst, list, s);
+        return launch_dependent(k_rows_pt<N>, dim3(count * PtRowShape<N>::BPI), PtRowShape<N>::TPB, st, inst, list, s);
     return cudaGetLastError();
 }
 
 // 16-column tiles when several solves fill the GPU; 4-column tiles (four times the blocks)
 // for one to three solves, where the launch would otherwise cover a few SMs.
 template <int N>
-static cudaError_t launch_cols_t(const InstDesc *inst, const int *list, int count, cudaStream_t st) {
+static cudaError_t launch_cols_t(const InstDesc *inst, const int *list, int count, int s, cudaStream_t st) {
     constexpr int G = LineShape<N>::G;
     if (count <= 0) return cudaSuccess;
     if (count >= 4)
-        k_cols<N, 16><<<dim3(count * (N / 16), 2), 16 * G, 0, st>>>(inst, list);
+        k_cols<N, 16><<<dim3(count * (N / 16), 2), 16 * G, 0, st>>>(inst, list, s);
     else
-        k_cols<N, 4><<<dim3(count * (N / 4), 2), 4 * G, 0, st>>>(inst, list);
+        return launch_dependent(k_cols<N, 4>, dim3(count * (N / 4), 2), 4 * G, st, inst, list, s);
     return cudaGetLastError();
 }
 
@@ -440,13 +443,13 @@ cudaError_t launch_rows(int n, const InstDesc *inst, const int *list, int count,
     }
 }
 
-cudaError_t launch_cols(int n, const InstDesc *inst, const int *list, int count, cudaStream_t st) {
+cudaError_t launch_cols(int n, const InstDesc *inst, const int *list, int count, int s, cudaStream_t st) {
     switch (n) {
-        case 16: return launch_cols_t<16>(inst, list, count, st);
-        case 32: return launch_cols_t<32>(inst, list, count, st);
-        case 64: return launch_cols_t<64>(inst, list, count, st);
-        case 128: return launch_cols_t<128>(inst, list, count, st);
-        case 256: return launch_cols_t<256>(inst, list, count, st);
+        case 16: return launch_cols_t<16>(inst, list, count, s, st);
+        case 32: return launch_cols_t<32>(inst, list, count, s, st);
+        case 64: return launch_cols_t<64>(inst, list, count, s, st);
+        case 128: return launch_cols_t<128>(inst, list, count, s, st);
+        case 256: return launch_cols_t<256>(inst, list, count, s, st);
         default: return cudaErrorInvalidValue;
     }
 }

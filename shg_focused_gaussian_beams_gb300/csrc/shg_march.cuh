@@ -150,4 +150,26 @@ __device__ __forceinline__ void rk4_point(float2 &P, float2 &S, float4 c, const 
     S = make_float2(fmaf(accs.x, d.dz6, S.x), fmaf(accs.y, d.dz6, S.y));
 }
 
+// The passes of a z step form a chain, each reading what the one before it wrote. Launched with
+// programmatic serialisation, a pass starts while its predecessor drains, fetches what no pass
+// writes (propagator, coefficients) and waits here for the predecessor's results. Measured in a
+// graph: one 256 x 256 x 400 march (two launches per z step) 2.63 -> 2.39 ms, its gradient 8.78 -> 8.41.
+// Letting the next pass start before this one ends (launch_dependents at its start) takes the SMs it
+// needs: 3.52 ms.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*k)(P...), dim3 grid, int threads, cudaStream_t st, A... a) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, P(a)...);
+}
+
 }  // namespace shg

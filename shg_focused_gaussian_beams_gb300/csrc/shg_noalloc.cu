@@ -160,7 +160,7 @@ extern "C" int shg_cwes_noalloc(const shg_config *cfg, float temp, const void *p
     const int K = cfg->nz - 1;
     for (int s = 0; s <= K; ++s) {
         NOALLOC_CUDA(launch_rows(n, d_desc, d_list, 1, s, st));
-        if (s < K) NOALLOC_CUDA(launch_cols(n, d_desc, d_list, 1, st));
+        if (s < K) NOALLOC_CUDA(launch_cols(n, d_desc, d_list, 1, s, st));
     }
     if (eta) {
         double acc[4] = {0, 0, 0, 0};

@@ -119,8 +119,12 @@ __device__ __forceinline__ void rows_body(const InstDesc &d, int line, int t, in
 // The column pass of k_cols for column x of field f (0 pump, 1 SH) of solve d, lane t of the
 // column's G lanes; the TC columns of a group transpose through sc (interleaved, stride TC)
 // and synchronise the block (BS) or, when the group is one warp, the warp.
-template <int N, int TC, bool BS, bool CG = false>
-__device__ __forceinline__ void cols_body(const InstDesc &d, int x, int f, int t, float2 *sc, const float2 *tab) {
+struct NoWait {
+    __device__ void operator()() const {}
+};
+template <int N, int TC, bool BS, bool CG = false, class Wait = NoWait>
+__device__ __forceinline__ void cols_body(const InstDesc &d, int x, int f, int t, float2 *sc, const float2 *tab,
+                                          Wait wait = Wait()) {
     constexpr int G = LineShape<N>::G, E = N / G;
     float2 *F = f == 0 ? d.P : d.S;
     const float2 *__restrict__ H = f == 0 ? d.Hp : d.Hs;
@@ -128,6 +132,7 @@ __device__ __forceinline__ void cols_body(const InstDesc &d, int x, int f, int t
     // propagator values first: their latency overlaps the transform
     float2 h[E];
     hprop_load<N>(H, x, t, h);
+    wait();
     float2 v[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) v[j] = ld_field<CG>(&SHG_AT(F, (size_t)(t + G * j) * N + x, NN, kChkColsGlobal));

@@ -402,7 +402,7 @@ int ThermalSolve::cwes(float power, float waist, float focal) {
     const int *list0 = reinterpret_cast<const int *>(acc_ + 4);
     for (int s = 0; s <= nz_; ++s) {
         TH_CUDA(launch_rows_th(n_, d_desc_, th_, s, st_));
-        if (s < nz_) TH_CUDA(launch_cols(n_, d_desc_, list0, 1, st_));
+        if (s < nz_) TH_CUDA(launch_cols(n_, d_desc_, list0, 1, s, st_));
     }
     return SHG_OK;
 }
