@@ -6,8 +6,8 @@
 // columns [rank R, rank R + R) (column phase, read and written through distributed shared
 // memory); a cluster barrier separates the phases. Against the resident cluster march
 // (shg_resident.cuh, R * G threads per CTA, each carrying N / G points through both RK4
-// calls) every CTA here has 512 threads: the line transforms run on 2 R G of them and the
-// two RK4 calls on all of them, R N / 512 points each, through the shared field rows. The
+// calls) every CTA here has 512 threads (fewer where it has fewer points): the line transforms run on 2 R G of
+// them and the two RK4 calls on all of them, R N / 512 points each, through the shared field rows. The
 // arithmetic is that of the streaming row and column passes (k_rows_pt, k_cols in
 // shg_march.cu): the same transforms, RK4 and propagator products in the same order, so
 // the output fields are bit-identical. Meant for lone solves (the march's latency is set by
@@ -36,7 +36,7 @@ struct CptShape {
     static constexpr int CS = CS_;
     static constexpr int G = LineShape<N>::G, E = N / G;
     static constexpr int R = N / CS;                   // rows (and columns) per CTA
-    static constexpr int TPB = 512;
+    static constexpr int TPB = R * N < 512 ? R * N : 512;
     static constexpr int PTS = R * N / TPB;            // points per thread in the pointwise phase
     static constexpr int XF = 2 * R * G;               // transform threads (both fields' lines)
     static constexpr int TC = 32 / G;                  // columns per warp in the column phase
@@ -259,7 +259,8 @@ static cudaError_t launch_cpt_t(const InstDesc *inst, const int *list, int count
 // 3.04 against 2.70.)
 int cluster_pt_sizes(int n, int *out) {
     switch (n) {
-        case 64: out[0] = 8, out[1] = 4; return 2;
+        case 32: out[0] = 4, out[1] = 2, out[2] = 1; return 3;
+        case 64: out[0] = 16, out[1] = 8, out[2] = 4; return 3;
         case 128: out[0] = 16, out[1] = 8; return 2;
         case 256: out[0] = 16; return 1;
         default: return 0;
@@ -269,6 +270,10 @@ int cluster_pt_sizes(int n, int *out) {
 cudaError_t prepare_cluster_pt(int n, int cs, int *max_clusters) {
     *max_clusters = 0;
     switch (n * 100 + cs) {
+        case 3204: return prepare_cpt_t<32, 4>(max_clusters);
+        case 3202: return prepare_cpt_t<32, 2>(max_clusters);
+        case 3201: return prepare_cpt_t<32, 1>(max_clusters);
+        case 6416: return prepare_cpt_t<64, 16>(max_clusters);
         case 6408: return prepare_cpt_t<64, 8>(max_clusters);
         case 6404: return prepare_cpt_t<64, 4>(max_clusters);
         case 12816: return prepare_cpt_t<128, 16>(max_clusters);
@@ -281,6 +286,10 @@ cudaError_t prepare_cluster_pt(int n, int cs, int *max_clusters) {
 cudaError_t launch_cluster_pt(int n, int cs, const InstDesc *inst, const int *list, int count, cudaStream_t st) {
     if (count < 1) return cudaErrorInvalidValue;
     switch (n * 100 + cs) {
+        case 3204: return launch_cpt_t<32, 4>(inst, list, count, st);
+        case 3202: return launch_cpt_t<32, 2>(inst, list, count, st);
+        case 3201: return launch_cpt_t<32, 1>(inst, list, count, st);
+        case 6416: return launch_cpt_t<64, 16>(inst, list, count, st);
         case 6408: return launch_cpt_t<64, 8>(inst, list, count, st);
         case 6404: return launch_cpt_t<64, 4>(inst, list, count, st);
         case 12816: return launch_cpt_t<128, 16>(inst, list, count, st);

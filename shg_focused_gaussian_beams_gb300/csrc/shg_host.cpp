@@ -224,11 +224,12 @@ int ensure_twiddles(int device) {
 }
 
 // The cluster march of a class: the largest cluster size of which the class's solves fit in one wave,
-// otherwise the largest that fits at all (g == 0: none); *mc: how many fit at once. A z step of 64 x 64
-// takes 3.4 us on eight CTAs (up to 18 solves) and 4.8 on four (37): 24 solves of 200 slices 1.25 ms by
-// resident clusters of four CTAs, 0.96 so; 128 x 128 on eight CTAs (9 to 17 solves) 2.46 -> 1.89 ms.
+// otherwise the largest that fits at all (g == 0: none); *mc: how many fit at once. us per z step of a
+// wave by cluster size (solves that fit): 32 x 32 on four CTAs (36) 1.8, two (74) 2.3, one (152) 3.6,
+// resident march 3.9; 64 x 64 on sixteen (8) 2.5, eight (17) 3.1, four (37) 4.5, resident clusters of
+// four CTAs 6.0; 128 x 128 on sixteen (8) 6.2, eight (17) 9.1, resident 12.1.
 static ResidentVariant cluster_variant(int n, int count, int *mc) {
-    int sizes[2] = {0, 0};
+    int sizes[3] = {0, 0, 0};
     const int k = cluster_pt_sizes(n, sizes);
     ResidentVariant first{-1, 1, 0};
     int first_mc = 0;
@@ -794,7 +795,7 @@ class Batch {
             } else if (resident == 3) {
                 int mc = 0;
                 const ResidentVariant cv = cluster_variant(n, c.count, &mc);
-                if (cv.g < 1) {
+                if (n < 64 || cv.g < 1) {
                     set_error("set_schedule: the cluster march runs grids 64, 128 and 256 where a cluster fits");
                     return SHG_ERR_UNSUPPORTED;
                 }

@@ -76,9 +76,9 @@ bool line_length_supported(int n);
 
 // shg_cluster_pt.cu: the march of each of `count` solves (list[0..count)) in one
 // thread-block cluster of cs CTAs (one of cluster_pt_sizes), both fields in the cluster's shared
-// memory (n in {64, 128, 256}). prepare_cluster_pt: once per device, outside any capture;
+// memory (n in {32, 64, 128, 256}). prepare_cluster_pt: once per device, outside any capture;
 // max_clusters receives how many clusters fit at once (0: none).
-int cluster_pt_sizes(int n, int *out);  // up to 2
+int cluster_pt_sizes(int n, int *out);  // up to 3
 cudaError_t prepare_cluster_pt(int n, int cs, int *max_clusters);
 cudaError_t launch_cluster_pt(int n, int cs, const InstDesc *inst, const int *list, int count, cudaStream_t st);
 // shg_group.cu: the march of `njobs` solves (list[0..njobs)) by persistent groups of blocks with

@@ -34,3 +34,19 @@ def test_cluster_sizes_match_streaming(n, count):
     np.testing.assert_allclose(ec, es, rtol=1e-12, atol=0)
     for a, b in zip(fc, fs):
         assert np.array_equal(a, b)
+
+
+# sizes that the schedule call does not name: the variable fixes the kind, the count the cluster size
+@pytest.mark.parametrize("n,count", [(32, 1), (32, 36), (32, 40), (32, 74), (32, 80), (32, 160), (64, 8), (64, 9)])
+def test_small_grids_match_streaming(monkeypatch, n, count):
+    insts = [W.plain_instance(n, 2 + i % 4, 3.0 + i % 7, 1.0 + 0.1 * (i % 9), 50.0) for i in range(count)]
+    es, fs = _fields(insts, n, False)
+    monkeypatch.setenv("SHG_MARCH", f"{n}:cluster")
+    sw = Sweep(insts, crystal=W.CRYSTAL_QPM50)
+    assert "cluster march" in sw.schedule()
+    for _ in range(2):
+        ec, fc = sw.run(with_fields=True)
+    np.testing.assert_allclose(ec, es, rtol=1e-12, atol=0)
+    for a, b in zip(fc, fs):
+        assert np.array_equal(a, b)
+    sw.close()

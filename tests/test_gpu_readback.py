@@ -13,7 +13,7 @@ from shg_focused_gaussian_beams_gb300 import workloads as W  # noqa: E402
 from shg_focused_gaussian_beams_gb300.solver import Solver  # noqa: E402
 
 
-@pytest.mark.parametrize("n", [32, 64, 128])  # persistent grid, cluster march, persistent grid on split lanes
+@pytest.mark.parametrize("n", [32, 64, 128])  # cluster march, cluster march, persistent grid
 def test_powers_follow_the_last_run(n):
     inst = W.plain_instance(n, 12, 20.0, 2.84, 50.0)
 
