@@ -362,8 +362,13 @@ template <int N>
 static cudaError_t launch_adj_rows_bwd_t(const InstDesc *d, float2 *C, int s, int finish, int start,
                                          const float2 *Xn, const float2 *Wn, double *acc_fin, double *acc_start,
                                          cudaStream_t st) {
-    return launch_dependent(k_adj_rows_bwd<N>, dim3(AdjRowShape<N>::BPI), AdjRowShape<N>::TPB, st, d, C, s, finish,
-                            start, Xn, Wn, acc_fin, acc_start);
+    if (finish)
+        return launch_dependent(k_adj_rows_bwd<N>, dim3(AdjRowShape<N>::BPI), AdjRowShape<N>::TPB, st, d, C, s, finish,
+                                start, Xn, Wn, acc_fin, acc_start);
+    // the first pass of a segment: its stored states may be the last that the replay branch wrote
+    k_adj_rows_bwd<N><<<AdjRowShape<N>::BPI, AdjRowShape<N>::TPB, 0, st>>>(d, C, s, finish, start, Xn, Wn, acc_fin,
+                                                                            acc_start);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_adj_rows_fwd(int n, const InstDesc *d, float2 *A, int s, int finish, int start, const float2 *inP,
