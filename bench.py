@@ -212,8 +212,8 @@ def run_thermal_adjoint(args, count=64, n=256, nz=400, design_steps=20):
 
 
 def run_heat(args):
-    """Heat sweeps alone on the 256x256x400 THERMAL grid: one sweep per launch and K = 2, 3,
-    4 sweeps per launch (temporal blocking); algorithmic bytes 12 per voxel and sweep."""
+    """Heat sweeps alone on the 256x256x400 THERMAL grid by the single-sweep kernels (level 1) or two
+    sweeps per launch (levels 2 to 4); algorithmic bytes 12 per voxel and sweep."""
     inst = W.config_thermal_256()
     vox = inst.nx * inst.ny * inst.nz
     peak, kind = measured_hbm()
@@ -268,12 +268,13 @@ def run_thermal(args):
             "config": {"workload": "thermal256: 256x256x400, P=30 W, xi=2.84, 2000x1000 um cross-section, "
                                    "oven-surrounded faces at a seeded U(45,55) C", "t_oven": inst.temp},
             "jacobi_counts": counts, "voxel_sweeps_per_s": vox * sweeps / t,
-            "roofline": {"bound": "hbm", "kernel": "k_heat_tma<1,4> (one Jacobi sweep: TMA plane ring, 4 rows per "
-                                                   "consumer warp, 8-plane chunks)",
+            "roofline": {"bound": "hbm", "kernel": "k_heat_block (two Jacobi sweeps per launch on register "
+                                                   "tiles; figures per sweep)",
                          "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak, "peak_source": peak_kind, "ms_per_launch": 1e3 * per_sweep,
-                         "algorithmic_bytes_per_launch": 12.0 * vox, "traffic": heat_traffic(vox),
-                         "note": "CUDA events around 400 back-to-back sweeps on the launching stream"},
+                         "algorithmic_bytes_per_launch": 12.0 * vox, "traffic": None,
+                         "note": "CUDA events around 400 back-to-back sweeps on the launching stream; two sweeps per "
+                                 "pass move half of the 12 bytes per voxel and sweep"},
             "clocks": clk.summary(), "efficiency": s.efficiency()}
     # the workload's relative-residual stop rule (||dT|| / ||T|| < 1e-6, checked every 100 sweeps)
     s.set_jacobi_rule(1e-6, check_every=100)
@@ -436,13 +437,6 @@ def ncu_traffic(kernel):
             return json.load(f).get(kernel)
     except (OSError, ValueError):
         return None
-
-
-def heat_traffic(vox):
-    """DRAM bytes of one TMA-staged sweep over `vox` voxels from the committed ncu capture
-    (bytes per voxel of a 256x256x400 launch), or None."""
-    t = ncu_traffic("heat_tma<4>")
-    return None if t is None else t["bytes_per_voxel"] * vox
 
 
 def dist_setup(n_gpus):
