@@ -108,7 +108,7 @@ __device__ __forceinline__ void th_vjp_point(const float2 P, const float2 S, flo
 // with 256 threads. 1 and 2 shorten the chain of points that a thread works through, for batches
 // that leave the SMs room (row_shape).
 template <int N, int SHAPE>
-struct ThRowShape {
+struct ThPassShape {
     static constexpr int G = LineShape<N>::G, E = N / G;
     static constexpr int LMAX = (SHAPE == 2 ? 32 : 64) / G, LPB = LMAX < N ? LMAX : N;  // lines per field
     static constexpr int FT = LPB * G;                                           // transform threads per field
@@ -122,11 +122,11 @@ struct ThRowShape {
 // Roles of a thread: transform role (line of field f, lane t) and point role (points i of the
 // block's LPB * N, consecutive threads consecutive points).
 template <int N, int SHAPE>
-struct ThRow {
-    using Sh = ThRowShape<N, SHAPE>;
+struct ThPassRow {
+    using Sh = ThPassShape<N, SHAPE>;
     static constexpr int G = Sh::G, E = Sh::E, LPB = Sh::LPB, SC = Sh::SC;
     float2 *sm;
-    __device__ ThRow(float2 *s) : sm(s) {}
+    __device__ ThPassRow(float2 *s) : sm(s) {}
     __device__ static bool transforms() { return threadIdx.x < 2 * Sh::FT; }
     __device__ float2 *line() const { return sm + (threadIdx.x / G) * SC; }  // lines [0, LPB) pump, then SH
     __device__ static size_t row() {  // this thread's row in the solve's state (pump, then SH)
@@ -167,17 +167,17 @@ struct ThRow {
 // save_x. With sn >= 0 RK4_th of step sn (its first call) and the start of its diffraction in A;
 // otherwise the state to out. Null pointers skip their stores, and the RK4 that nothing reads.
 template <int N, int SHAPE>
-__global__ void __launch_bounds__(ThRowShape<N, SHAPE>::TPB, ThRowShape<N, SHAPE>::BLOCKS)
+__global__ void __launch_bounds__(ThPassShape<N, SHAPE>::TPB, ThPassShape<N, SHAPE>::BLOCKS)
     k_th_rows_fwd(float2 *A0, const float2 *inP, const float2 *inS, size_t stride, float2 *save_w, float2 *save_x,
                   float2 *out, const float4 *__restrict__ coef, int K, int sp, int sn,
                   const InstDesc *__restrict__ dd) {
-    using Sh = ThRowShape<N, SHAPE>;
+    using Sh = ThPassShape<N, SHAPE>;
     __shared__ float2 sm[2 * Sh::LPB * Sh::SC];
     constexpr int NN = N * N, P = Sh::LPB * N;
     const int b = blockIdx.y, base = blockIdx.x * P;  // this block's points of a field
     const InstDesc &d = dd[b];
     const float2 *__restrict__ tab = g_twiddle + N;
-    const ThRow<N, SHAPE> rw(sm);
+    const ThPassRow<N, SHAPE> rw(sm);
     float2 *A = A0 + (size_t)b * 2 * NN;
     const size_t o = (size_t)b * 2 * NN + base;
     const float4 *__restrict__ cp = coef + ((size_t)b * K + (sp < 0 ? 0 : sp)) * NN + base;
@@ -237,16 +237,16 @@ __global__ void __launch_bounds__(ThRowShape<N, SHAPE>::TPB, ThRowShape<N, SHAPE
 // RK4_th^T of step sb at its second call's input Wb and the start of its adjoint diffraction in C,
 // otherwise the cotangent to C.
 template <int N, int SHAPE>
-__global__ void __launch_bounds__(ThRowShape<N, SHAPE>::TPB, ThRowShape<N, SHAPE>::BLOCKS)
+__global__ void __launch_bounds__(ThPassShape<N, SHAPE>::TPB, ThPassShape<N, SHAPE>::BLOCKS)
     k_th_rows_bwd(float2 *C0, const float2 *__restrict__ Xa, const float2 *__restrict__ Wb,
                   const float4 *__restrict__ coef, int K, int sa, int sb, const InstDesc *__restrict__ dd) {
-    using Sh = ThRowShape<N, SHAPE>;
+    using Sh = ThPassShape<N, SHAPE>;
     __shared__ float2 sm[2 * Sh::LPB * Sh::SC];
     constexpr int NN = N * N, P = Sh::LPB * N;
     const int b = blockIdx.y, base = blockIdx.x * P;
     const InstDesc &d = dd[b];
     const float2 *__restrict__ tab = g_twiddle + N;
-    const ThRow<N, SHAPE> rw(sm);
+    const ThPassRow<N, SHAPE> rw(sm);
     float2 *C = C0 + (size_t)b * 2 * NN;
     const size_t o = (size_t)b * 2 * NN + base;
     const float4 *__restrict__ ca = coef + ((size_t)b * K + (sa < 0 ? 0 : sa)) * NN + base;
@@ -345,7 +345,7 @@ cudaError_t launch_th_coef_table(const float *NP, const float *NS, const float *
 //    more          64^2 x 64  12.8/32.2  13.4/34.4  12.5/34.1     256^2 x 8   21.1/58.4  22.2/62.6  24.4/69.9
 template <int N>
 static int row_shape(int solves, int sms) {
-    const int blocks = solves * ThRowShape<N, 0>::BPI;
+    const int blocks = solves * ThPassShape<N, 0>::BPI;
     return blocks < sms ? 2 : blocks < 2 * sms ? 1 : 0;
 }
 
@@ -353,7 +353,7 @@ template <int N, int SHAPE>
 static cudaError_t launch_rows_fwd_s(float2 *A, const float2 *inP, const float2 *inS, size_t stride, float2 *save_w,
                                      float2 *save_x, float2 *out, const float4 *coef, int K, int sp, int sn,
                                      const InstDesc *d, int solves, cudaStream_t st) {
-    using Sh = ThRowShape<N, SHAPE>;
+    using Sh = ThPassShape<N, SHAPE>;
     return launch_dependent(k_th_rows_fwd<N, SHAPE>, dim3(Sh::BPI, solves), Sh::TPB, st, A, inP, inS, stride, save_w,
                             save_x, out, coef, K, sp, sn, d);
 }
@@ -372,7 +372,7 @@ static cudaError_t launch_rows_fwd_t(float2 *A, const float2 *inP, const float2 
 template <int N, int SHAPE>
 static cudaError_t launch_rows_bwd_s(float2 *C, const float2 *Xa, const float2 *Wb, const float4 *coef, int K, int sa,
                                      int sb, const InstDesc *d, int solves, cudaStream_t st) {
-    using Sh = ThRowShape<N, SHAPE>;
+    using Sh = ThPassShape<N, SHAPE>;
     return launch_dependent(k_th_rows_bwd<N, SHAPE>, dim3(Sh::BPI, solves), Sh::TPB, st, C, Xa, Wb, coef, K, sa, sb, d);
 }
 

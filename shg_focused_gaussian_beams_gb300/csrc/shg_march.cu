@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(RowShape<N>::TPB, N >= 128 ? 2 : 0) k_rows(con
 }
 
 // Row pass for one to three solves: the same work as k_rows with one thread per point.
-// Block = LPB lines x N threads; the row transforms run on 2 * LPB * G threads (pump lines
+// Block = LPB lines x N threads; the row transforms run on 2 * LPB * LW threads (pump lines
 // first, then SH lines), both RK4 calls on every thread for its point through a
 // shared-memory line buffer, so a lone solve occupies N * N threads instead of N * G.
 template <int N>

@@ -427,7 +427,7 @@ __device__ __forceinline__ void block_add_double_th(double v, double *dst) {
 }
 
 // Block shape: LPB lines, one thread per point (LPB * N threads). The row transforms run on
-// 2 * LPB * G threads (the pump's lines on the first LPB * G, the SH's on the next), the
+// 2 * LPB * LW threads (the pump's lines on the first LPB * LW, the SH's on the next), the
 // per-point RK4 and heat source on all threads with the point in natural x order, so the
 // per-voxel loads are coalesced and the coupling arithmetic is spread over N threads per
 // line instead of G.
@@ -438,7 +438,7 @@ struct ThRowShape {
     static constexpr int TPB = LPB * N;
     static constexpr int BPI = N / LPB;
     static_assert(LPB >= 1 && N % LPB == 0, "whole lines per block");
-    static constexpr int LW = RowLanes<N, false>::LW, FFT_THREADS = LPB * LW;  // per field (split lanes)
+    static constexpr int LW = RowLanes<N, false>::LW, FFT_THREADS = LPB * LW;  // per field
     static_assert(FFT_THREADS % 32 == 0 && 2 * FFT_THREADS <= TPB, "transform threads fill whole warps");
 };
 
