@@ -174,14 +174,15 @@ __device__ __forceinline__ float div_const(float a, float d, float r, int fast) 
 // K = kh + kl to 48 bits. The sum and product are carried as pairs of floats, which is within
 // 2^-44 (|s| + |K|) |D| of the exact value, as the double result is; where the float roundings of both
 // ends of that interval agree, that float is the answer, else (one in a million, and infinities
-// and NaN) the doubles decide. About 15 float instructions against five FP64 ones at 1/64 rate:
-// on the faces' threads these were a third of a step of the open-top sweep.
+// and NaN) the doubles decide. The pairs are exact to 2^-150 only, so the interval is widened by 2^-126:
+// products below 2^-102, whose own ulp is less, go to the doubles. About 15 float instructions against
+// five FP64 ones at 1/64 rate: on the faces' threads these were a third of a step of the open-top sweep.
 __device__ __forceinline__ float edge_round(float s, double K, float kh, float kl, float D) {
     const float h = __fadd_rn(s, kh), t = __fsub_rn(h, s);
     const float e = __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(h, t)), __fsub_rn(kh, t)), kl);  // s + kh + kl - h
     const float p = __fmul_rn(h, D);
     const float lo = __fmaf_rn(e, D, __fmaf_rn(h, D, -p));
-    const float d = __fmul_rn(__fmul_rn(__fadd_rn(fabsf(s), fabsf(kh)), fabsf(D)), 0x1p-44f);
+    const float d = __fmaf_rn(__fmul_rn(__fadd_rn(fabsf(s), fabsf(kh)), fabsf(D)), 0x1p-44f, 0x1p-126f);
     const float a = __fadd_rn(p, __fadd_rn(lo, d)), b = __fadd_rn(p, __fsub_rn(lo, d));
     float r = a;
     if (!(a == b)) r = __double2float_rn(__dmul_rn(__dadd_rn((double)s, K), (double)D));
