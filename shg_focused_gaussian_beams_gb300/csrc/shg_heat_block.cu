@@ -119,43 +119,30 @@ struct Range {
     __device__ __forceinline__ bool out() const { return !(lo >= 0x1p-60f && hi < 0x1p99f); }
 };
 
-// Four voxels (x .. x+3, y) of plane z of any class, from the shared plane z (pl: this vector,
-// pm / pp: rows y-1 / y+1, left / right: the offsets of the outer x neighbours) and the values
-// at z-1, z+1: the faces' formulas, the voxels the reference never writes (kept), and
-// numerators outside the verified range of the corrected products. Out of line: the interior
-// of a grid does not come here.
-template <int BC>
-__device__ __noinline__ V4 update4_any(const HeatCoef &c, const HeatBlockGrid &g, int x, int y, int z, const float *pl,
-                                       const float *pm, const float *pp, V4 zm, V4 zp, V4 q, int left, int right) {
-    const float2 a01 = unpack2(zm.a), a23 = unpack2(zm.b), b01 = unpack2(zp.a), b23 = unpack2(zp.b);
-    const float2 q01 = unpack2(q.a), q23 = unpack2(q.b);
-    const float cv[6] = {pl[left], pl[0], pl[1], pl[2], pl[3], pl[right]};
-    const float a[4] = {a01.x, a01.y, a23.x, a23.y}, b[4] = {b01.x, b01.y, b23.x, b23.y};
-    const float qk[4] = {q01.x, q01.y, q23.x, q23.y};
-    float o[4];
-    const bool zface = z == 0 || z == g.nz - 1, yint = y > 0 && y < g.ny - 1, ytop = BC == 0 && y == g.ny - 1;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const bool xint = x + e > 0 && x + e < g.nx - 1;
-        if (zface && yint && xint) {  // the bulk of the z faces
-            float s = __fadd_rn(z == 0 ? b[e] : a[e], __fmul_rn(c.az, __fadd_rn(cv[e + 2], cv[e])));
-            s = __fadd_rn(s, __fmul_rn(c.bz, __fadd_rn(pp[e], pm[e])));
-            s = __fadd_rn(s, c.tinfBiz);
-            o[e] = div_const(s, c.den_z, c.rden_z, c.fast_face);
-        } else if (ytop && xint && !zface) {  // the bulk of the top face
-            float s = __fadd_rn(pm[e], __fmul_rn(c.ay, __fadd_rn(cv[e + 2], cv[e])));
-            s = __fadd_rn(s, __fmul_rn(c.by, __fadd_rn(b[e], a[e])));
-            s = __fadd_rn(s, c.tinfBiy);
-            o[e] = div_const(s, c.den_y, c.rden_y, c.fast_face);
-        } else {
-            float v;
-            o[e] = heat_voxel<BC>(c, x + e, y, z, g.nx, g.ny, g.nz, cv[e], cv[e + 2], pm[e], pp[e], a[e], b[e], qk[e], v)
-                       ? v
-                       : cv[e + 1];
-        }
-    }
-    return {pack2(o[0], o[1]), pack2(o[2], o[3])};
+__device__ __forceinline__ u64 div2_any(u64 s, float d, float r, int fast) {
+    const float2 v = unpack2(s);
+    return pack2(div_any(v.x, d, r, fast), div_any(v.y, d, r, fast));
 }
+// Magnitudes seen where zeros may be among them: with the sign rotated to the bottom and less one, +0
+// is the largest of unsigned values, -0 the smallest (its quotient is -0, that of a corrected product
+// +0).
+struct RangeZero {
+    unsigned lo;
+    float hi;
+    __device__ __forceinline__ void add(u64 s) {
+        const float2 v = unpack2(s);
+        const unsigned a = __float_as_uint(v.x), b = __float_as_uint(v.y);
+        lo = min(lo, min(__funnelshift_l(a, a, 1) - 1u, __funnelshift_l(b, b, 1) - 1u));
+        hi = max_abs3(hi, v.x, v.y);
+    }
+    __device__ __forceinline__ void add(V4 v) { add(v.a), add(v.b); }
+    // +0 or a magnitude in [2^(elo - 127), top)
+    __device__ __forceinline__ bool in(unsigned elo, float top) const { return lo >= (elo << 24) - 1u && hi < top; }
+    // Temperatures: sums of two are +0 or in [2^-100, 2^100).
+    __device__ __forceinline__ bool out() const { return !in(50u, 0x1p99f); }
+    // Numerators: as the corrected products were verified for.
+    __device__ __forceinline__ bool ok() const { return in(kDivExpLo, 0x1p101f); }
+};
 
 struct DivConst {  // reciprocals, negated divisors and the final factor, both halves alike
     u64 rx, ndx, ry, ndy, rz, ndz, l2;
@@ -182,18 +169,31 @@ __device__ __forceinline__ V4 interior4(const DivConst &d, const Sums &s, V4 sz,
     return o;
 }
 
-// A face formula for four voxels: (n + a s1 + b s2 + t) / den, n the inward neighbour. Scalar
-// products and sums: the packed forms carry no promise against contraction.
-__device__ __forceinline__ V4 face4(V4 n, u64 s1a, u64 s1b, u64 s2a, u64 s2b, float a, float b, float t, float den,
-                                    float rden) {
-    const float2 n01 = unpack2(n.a), n23 = unpack2(n.b), u01 = unpack2(s1a), u23 = unpack2(s1b), w01 = unpack2(s2a),
-                 w23 = unpack2(s2b);
-    auto f = [&](float n1, float u, float w) {
-        return __fadd_rn(__fadd_rn(__fadd_rn(n1, __fmul_rn(a, u)), __fmul_rn(b, w)), t);
+// The same for numerators of any magnitude, out of line: only values below 2^-77 (a Gaussian's
+// underflowing tails beside zeros), infinities and -0 come here.
+__device__ __noinline__ V4 interior4_any(const HeatCoef &c, Sums s, V4 sz, V4 q) {
+    auto half = [&](u64 x, u64 y, u64 z, u64 q2) {
+        return mul2(twice(c.L2), add2(add2(add2(div2_any(x, c.dx2, c.rdx2, c.fast_div),
+                                                div2_any(y, c.dy2, c.rdy2, c.fast_div)),
+                                           div2_any(z, c.dz2, c.rdz2, c.fast_div)), q2));
     };
-    const u64 r = twice(rden), nd = twice(-den);
-    return {div2(pack2(f(n01.x, u01.x, w01.x), f(n01.y, u01.y, w01.y)), r, nd),
-            div2(pack2(f(n23.x, u23.x, w23.x), f(n23.y, u23.y, w23.y)), r, nd)};
+    return {half(s.xa, s.ya, sz.a, q.a), half(s.xb, s.yb, sz.b, q.b)};
+}
+
+// The z faces' formula for four voxels: (n + az s1 + bz s2 + t) / den_z, n the inward neighbour, s1
+// and s2 the sums of the x and y neighbours. Scalar products and sums: the packed forms carry no
+// promise against contraction. ANY: numerators of any magnitude.
+template <bool ANY>
+__device__ __forceinline__ V4 face4(const HeatCoef &c, V4 n, const Sums &s) {
+    auto f = [&](u64 n2, u64 s1, u64 s2) {
+        const float2 m = unpack2(n2), u = unpack2(s1), w = unpack2(s2);
+        auto g = [&](float n1, float u1, float w1) {
+            return __fadd_rn(__fadd_rn(__fadd_rn(n1, __fmul_rn(c.az, u1)), __fmul_rn(c.bz, w1)), c.tinfBiz);
+        };
+        const u64 v = pack2(g(m.x, u.x, w.x), g(m.y, u.y, w.y));
+        return ANY ? div2_any(v, c.den_z, c.rden_z, c.fast_face) : div2(v, twice(c.rden_z), twice(-c.den_z));
+    };
+    return {f(n.a, s.xa, s.ya), f(n.b, s.xb, s.yb)};
 }
 
 // mask ? a : b, bitwise (masks all ones or zero)
@@ -205,8 +205,8 @@ __device__ __forceinline__ float blend(unsigned m, float a, float b) {
 
 // BC 0: the voxel of the four that lies on the face x = 0 (left) or x = NX-1, of a row inside
 // the grid in y: the face formula away from the z faces (zs: sums of the z neighbours), else
-// the vertical edge's (zs: the inward z neighbours).
-template <bool ZFACE>
+// the vertical edge's (zs: the inward z neighbours). ANY: numerators of any magnitude.
+template <bool ZFACE, bool ANY = false>
 __device__ __forceinline__ float x_face(const HeatCoef &c, V4 cc, const Sums &s, V4 zs, bool left) {
     const float2 zl = unpack2(zs.a), zr = unpack2(zs.b), yl = unpack2(s.ya), yr = unpack2(s.yb);
     const float tx = left ? unpack2(cc.a).y : unpack2(cc.b).x;  // inward x neighbour
@@ -217,12 +217,13 @@ __device__ __forceinline__ float x_face(const HeatCoef &c, V4 cc, const Sums &s,
     float f = __fadd_rn(tx, __fmul_rn(c.ax, yy));
     f = __fadd_rn(f, __fmul_rn(c.bx, zz));
     f = __fadd_rn(f, c.tinfBix);
+    if (ANY) return div_any(f, c.den_x, c.rden_x, c.fast_face);
     const float w = f * c.rden_x;
     return fmaf(fmaf(-w, c.den_x, f), c.rden_x, w);
 }
 
 // BC 0: four voxels of the top face y = NY-1, its edges and corners included (zs as above).
-template <bool ZFACE>
+template <bool ZFACE, bool ANY = false>
 __device__ __forceinline__ V4 top_row(const HeatCoef &c, V4 cc, const Sums &s, V4 ym, V4 zs, bool left, bool right) {
     const float2 c01 = unpack2(cc.a), c23 = unpack2(cc.b), m01 = unpack2(ym.a), m23 = unpack2(ym.b);
     const float2 x01 = unpack2(s.xa), x23 = unpack2(s.xb), z01 = unpack2(zs.a), z23 = unpack2(zs.b);
@@ -240,7 +241,7 @@ __device__ __forceinline__ V4 top_row(const HeatCoef &c, V4 cc, const Sums &s, V
             f = __fadd_rn(f, __fmul_rn(c.by, z[i]));
             f = __fadd_rn(f, c.tinfBiy);
             const float w = f * c.rden_y;
-            o[i] = fmaf(fmaf(-w, c.den_y, f), c.rden_y, w);
+            o[i] = ANY ? div_any(f, c.den_y, c.rden_y, c.fast_face) : fmaf(fmaf(-w, c.den_y, f), c.rden_y, w);
         }
     }
     if (ZFACE) {
@@ -253,23 +254,20 @@ __device__ __forceinline__ V4 top_row(const HeatCoef &c, V4 cc, const Sums &s, V
     return {pack2(left ? e : o[0], o[1]), pack2(o[2], right ? e : o[3])};
 }
 
-// vx (a power of two, at most 32) vectors per region row: rows start at warp boundaries or
-// share a warp, so x neighbours across a row's ends belong to no stored voxel.
-template <int BC, int K, int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS)
-    k_heat_block(float *__restrict__ Tf, const float *__restrict__ Ti, const float *__restrict__ QK,
-                 const __grid_constant__ HeatCoef c, const __grid_constant__ HeatBlockGrid g) {
+// Planes [z0, z1) of a block's tile. vx (a power of two, at most 32) vectors per region row: rows start at warp
+// boundaries or share a warp, so x neighbours across a row's ends belong to no stored voxel.
+// ORDINARY: returns the first plane that is not stored, z1 unless a value was out of range (then with no
+// copy in flight). Otherwise values of any kind.
+template <int BC, int K, int THREADS, bool ORDINARY>
+__device__ __forceinline__ int heat_chunk(float *__restrict__ Tf, const float *__restrict__ Ti,
+                                          const float *__restrict__ QK, const HeatCoef &c, const HeatBlockGrid &g,
+                                          const int z0, const int z1) {
     static_assert(K <= kMaxLevels && K <= kRing - kAhead, "the Q/k ring holds the planes of K levels");
-    // Short chunks: the next sweep's blocks may start as soon as all of these have, so that their
-    // set-up up to their own wait overlaps this launch's last planes. Of long ones it takes SM
-    // slots for nothing (256x256x400 oven 48.4 us per sweep with it, 47.8 without).
-    if (g.zc <= 16) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int R = kRows, PL = plane_floats(THREADS, R);
     extern __shared__ __align__(16) float hb_smem[];
     const int vx = g.vx, rows = R * (THREADS / vx), row = 4 * vx;
     const int v = threadIdx.x & (vx - 1), r = R * (threadIdx.x / vx);
     const int x = (int)blockIdx.x * g.txi - g.xh + 4 * v, y = (int)blockIdx.y * g.tyi - g.yh + r;
-    const int z0 = (int)blockIdx.z * g.zc, z1 = min(g.nz, z0 + g.zc);
     const size_t sxy = (size_t)g.nx * g.ny;
     // this thread's first vector in shared plane 0, and the rows above and below its own;
     // planes: input ring, Q/k ring, levels 1..K-1
@@ -278,7 +276,6 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
     const bool xin = x >= 0 && x < g.nx;
     const bool xst = xin && x >= (int)blockIdx.x * g.txi && x < ((int)blockIdx.x + 1) * g.txi;
     const int ylo = (int)blockIdx.y * g.tyi, yhi = min(g.ny, ylo + g.tyi);
-    const int left = v == 0 ? 0 : -1, right = v == vx - 1 ? 3 : 4;  // x neighbours (own value at a region's end: not used)
     bool in[R], st[R];
     bool top[R];                     // BC 0: the row is on the top face
     unsigned keep[R], kl[R], kr[R];  // voxels that are kept: the middle two, the first, the last
@@ -343,13 +340,16 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
                         twice(c.L2)};
     // Q/k is checked against 2^60 beside the temperatures, so that a value computed in the
     // running step, whose range the others learn at the next barrier, is below 2^100 too
-    Range seen{c.fast_div && c.fast_face && c.L2 < 0x1p30f ? 1.0f : 0.0f, 1.0f};
+    auto verified = [&] { return c.fast_div && c.fast_face && c.L2 < 0x1p30f; };
+    Range seen{verified() ? 1.0f : 0.0f, 1.0f};         // of the ordinary chunk
+    RangeZero seen0{verified() ? ~0u : 0u, 1.0f};  // of the other
     float qhi = 0.0f;
 
     // Arrival of plane p (ring slot s): this thread's values, then the barrier that orders the
     // previous step's level planes and plane p - 1, and tells every thread whether a value it
     // may read was out of range.
-    auto arrive = [&](int s) -> bool {
+    auto arrive = [&](auto Mode, int s) -> bool {
+        constexpr bool ZEROS = decltype(Mode)::value > 0;
         cp_async_wait<kAhead - 1>();
         const V4 q[R] = {ld4(sm + (kRing + s) * PL), ld4(sm1 + (kRing + s) * PL)};
         cur[0] = ld4(sm + s * PL);
@@ -359,11 +359,12 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             if (!in[k]) cur[k] = zm0[k] = ones;
-            seen.add(cur[k]);
+            if (ZEROS) seen0.add(cur[k]);
+            else seen.add(cur[k]);
             const float2 a = unpack2(q[k].a), b = unpack2(q[k].b);
             qhi = max_abs3(max_abs3(qhi, a.x, a.y), b.x, b.y);
         }
-        const bool bad = __syncthreads_or(seen.out() || !(qhi < 0x1p60f));
+        const bool bad = __syncthreads_or((ZEROS ? seen0.out() : seen.out()) || !(qhi < 0x1p60f));
         fetch((s + kAhead) % kRing);
         return bad;
     };
@@ -391,9 +392,10 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
     // Q/k of plane p - t: fetched with plane p - t + 1
     auto heat = [](int s, int t) { return kRing + (s - t + 1 + kRing) % kRing; };
 
-    // Step p with all values in range. Levels outside their range of planes compute on what
-    // they have; no stored voxel sees the result.
-    auto body = [&](int s, int p) {
+    // Step p: with all values in range (MODE 0), zeros among them (1), or values of any kind (2). Levels
+    // outside their range of planes compute on what they have; no stored voxel sees the result.
+    auto body = [&](auto Mode, int s, int p) {
+        constexpr int MODE = decltype(Mode)::value;
         sfor<K>([&](auto T) {
             constexpr int t = decltype(T)::value + 1;
             const int z = p - t;
@@ -413,26 +415,36 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
             auto lateral = [&](auto Z, int k, V4 zs) {
                 constexpr bool ZF = decltype(Z)::value;
                 if (xface) {
-                    const float e = x_face<ZF>(c, cc[t - 1][k], sums[k], zs, x == 0);
+                    const float e = x_face<ZF, (MODE > 0)>(c, cc[t - 1][k], sums[k], zs, x == 0);
                     const float2 o01 = unpack2(nw[k].a), o23 = unpack2(nw[k].b);
                     nw[k] = {pack2(x == 0 ? e : o01.x, o01.y), pack2(o23.x, x == 0 ? o23.y : e)};
                 }
                 if (top[k])
-                    nw[k] = top_row<ZF>(c, cc[t - 1][k], sums[k], k == 0 ? ym : cc[t - 1][0], zs, x == 0, x + 4 == g.nx);
+                    nw[k] = top_row<ZF, (MODE > 0)>(c, cc[t - 1][k], sums[k], k == 0 ? ym : cc[t - 1][0], zs, x == 0, x + 4 == g.nx);
             };
             if (z != 0 && z != g.nz - 1) {
 #pragma unroll
                 for (int k = 0; k < R; ++k) {
                     const V4 sz = {add2(cur[k].a, zm[k].a), add2(cur[k].b, zm[k].b)};
-                    nw[k] = interior4(d, sums[k], sz, ld4((k ? sm1 : sm) + heat(s, t) * PL));
+                    const V4 q = ld4((k ? sm1 : sm) + heat(s, t) * PL);
+                    bool ok = true;
+                    // this thread's own value of the level below, of this step, may be of any kind: the
+                    // others learn of it at the next barrier
+                    if (MODE == 1 && t > 1) ok = !seen0.out();
+                    if (MODE == 2) {
+                        RangeZero n{verified() ? ~0u : 0u, 0.0f};
+                        n.add(sums[k].xa), n.add(sums[k].xb), n.add(sums[k].ya), n.add(sums[k].yb);
+                        n.add(sz);
+                        ok = n.ok();
+                    }
+                    nw[k] = ok ? interior4(d, sums[k], sz, q) : interior4_any(c, sums[k], sz, q);
                     if (BC == 0) lateral(std::false_type{}, k, sz);
                 }
             } else {
 #pragma unroll
                 for (int k = 0; k < R; ++k) {
                     const V4 zn = z == 0 ? cur[k] : zm[k];
-                    nw[k] = face4(zn, sums[k].xa, sums[k].xb, sums[k].ya, sums[k].yb, c.az, c.bz, c.tinfBiz, c.den_z,
-                                  c.rden_z);
+                    nw[k] = face4<(MODE > 0)>(c, zn, sums[k]);
                     if (BC == 0) lateral(std::true_type{}, k, zn);
                 }
             }
@@ -442,7 +454,8 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
                 const float2 o01 = unpack2(nw[k].a), o23 = unpack2(nw[k].b);
                 nw[k].a = pack2(blend(kl[k], w01.x, o01.x), blend(keep[k], w01.y, o01.y));
                 nw[k].b = pack2(blend(keep[k], w23.x, o23.x), blend(kr[k], w23.y, o23.y));
-                if (t < K) seen.add(nw[k]);
+                if (t < K && MODE == 0) seen.add(nw[k]);
+                if (t < K && MODE == 1) seen0.add(nw[k]);
             }
             if (t == K) store(z, nw);
 #pragma unroll
@@ -453,32 +466,6 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
         });
         leave(s);
     };
-    // A step once a value was out of range: every voxel by its class, IEEE divisions.
-    auto body_any = [&](int s, int p) {
-#pragma unroll
-        for (int t = 1; t <= K; ++t) {
-            const int z = p - t;
-            const int pl = before(s, t) * PL;
-            V4 nw[R];
-#pragma unroll
-            for (int k = 0; k < R; ++k) {
-                nw[k] = cc[t - 1][k];
-                const V4 zm = t == 1 ? zm0[k] : ld4((k ? sm1 : sm) + older(s, t) * PL);
-                if (!keep[k] && z >= 0 && z < g.nz)
-                    nw[k] = update4_any<BC>(c, g, x, y + k, z, (k ? sm1 : sm) + pl, k ? sm + pl : smm + pl,
-                                            k ? smp + pl : sm1 + pl, zm, cur[k], ld4((k ? sm1 : sm) + heat(s, t) * PL),
-                                            left, right);
-            }
-            if (t == K) store(z, nw);
-#pragma unroll
-            for (int k = 0; k < R; ++k) {
-                cc[t - 1][k] = cur[k];
-                cur[k] = nw[k];
-            }
-        }
-        leave(s);
-    };
-
     // A step whose levels have nothing to compute yet: plane p only moves into place.
     auto skip = [&](int s) {
 #pragma unroll
@@ -487,45 +474,86 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
     };
     // The first step is one, and so is the second unless the chunk starts at the first slice: up to
     // half of the steps of the two- and four-plane chunks that small grids are cut into.
-    int p = plo, s = 0;
-    bool in_range = !arrive(0);
-    if (in_range) {
-        skip(0);
-        ++p;
-        s = 1;
-        in_range = !arrive(1);
-    }
-    if (in_range) {
-        if (plo > 0)
-            skip(1);
-        else
-            body(1, p);
-        if (++p > pend) return;
-        for (;;) {  // slots as constants: four steps to an iteration
-            s = 2;
-            if (arrive(2)) break;
-            body(2, p);
-            if (++p > pend) return;
-            s = 3;
-            if (arrive(3)) break;
-            body(3, p);
-            if (++p > pend) return;
-            s = 0;
-            if (arrive(0)) break;
-            body(0, p);
-            if (++p > pend) return;
-            s = 1;
-            if (arrive(1)) break;
-            body(1, p);
-            if (++p > pend) return;
+    constexpr std::integral_constant<int, 0> in_range{};
+    constexpr std::integral_constant<int, 1> zeros{};
+    constexpr std::integral_constant<int, 2> any{};
+    int p = plo;
+    if constexpr (ORDINARY) {
+        bool good = !arrive(in_range, 0);
+        if (good) {
+            skip(0);
+            ++p;
+            good = !arrive(in_range, 1);
+        }
+        if (good) {
+            if (plo > 0)
+                skip(1);
+            else
+                body(in_range, 1, p);
+            if (++p > pend) return z1;
+            for (;;) {  // slots as constants: four steps to an iteration
+                if (arrive(in_range, 2)) break;
+                body(in_range, 2, p);
+                if (++p > pend) return z1;
+                if (arrive(in_range, 3)) break;
+                body(in_range, 3, p);
+                if (++p > pend) return z1;
+                if (arrive(in_range, 0)) break;
+                body(in_range, 0, p);
+                if (++p > pend) return z1;
+                if (arrive(in_range, 1)) break;
+                body(in_range, 1, p);
+                if (++p > pend) return z1;
+            }
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        return max(z0, p - K);
+    } else {
+        int s = 0;
+        auto step = [&](auto Mode) {
+            if (p < plo + (plo > 0 ? 2 : 1))
+                skip(s);
+            else
+                body(Mode, s, p);
+            s = (s + 1) % kRing;
+            return ++p > pend;
+        };
+        // zeros and values down to 2^-77 first: the same step (the faces test their numerators); from the
+        // first value below that every numerator is tested
+        while (!arrive(zeros, s))
+            if (step(zeros)) return z1;
+        for (;;) {
+            if (step(any)) return z1;
+            arrive(any, s);
         }
     }
-    for (;;) {
-        body_any(s, p);
-        if (++p > pend) return;
-        s = (s + 1) % kRing;
-        arrive(s);
-    }
+}
+
+// The planes from a value out of range on. A crystal at 0 C has them: it holds zeros for good on the
+// faces that are never written, and heat spreads into the rest in small values. us per sweep with heat
+// down to 1e-20 from a zero crystal, open top / oven, ordinary temperatures in brackets: 64x64x200 8.1 (5.2)
+// / 5.9 (3.9), 256x256x400 83 (60) / 57 (46); with the heat of a Gaussian that underflows to denormals
+// 8.4 / 6.4, 128x128x200 19 (8.8) / 13 (6.3), 256x256x400 227 / 181, where a launch waits for its blocks
+// in the corners (the single-sweep kernels: 17 / 11, 23 / 16, 95 / 83). Out of line, so that it takes no
+// registers from the ordinary chunk (in line 64x64x200 open top 5.4 -> 5.5, out of line 5.2).
+template <int BC, int K, int THREADS>
+__device__ __noinline__ void heat_chunk_any(float *Tf, const float *Ti, const float *QK, const HeatCoef &c,
+                                            const HeatBlockGrid &g, int z0, int z1) {
+    heat_chunk<BC, K, THREADS, false>(Tf, Ti, QK, c, g, z0, z1);
+}
+
+template <int BC, int K, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS)
+    k_heat_block(float *__restrict__ Tf, const float *__restrict__ Ti, const float *__restrict__ QK,
+                 const __grid_constant__ HeatCoef c, const __grid_constant__ HeatBlockGrid g) {
+    // Short chunks: the next sweep's blocks may start as soon as all of these have, so that their
+    // set-up up to their own wait overlaps this launch's last planes. Of long ones it takes SM
+    // slots for nothing (256x256x400 oven 48.4 us per sweep with it, 47.8 without).
+    if (g.zc <= 16) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int z0 = (int)blockIdx.z * g.zc, z1 = min(g.nz, z0 + g.zc);
+    const int z = heat_chunk<BC, K, THREADS, true>(Tf, Ti, QK, c, g, z0, z1);
+    if (z < z1) heat_chunk_any<BC, K, THREADS>(Tf, Ti, QK, c, g, z, z1);
 }
 
 typedef void (*HeatBlockKernel)(float *, const float *, const float *, const HeatCoef, const HeatBlockGrid);

@@ -170,6 +170,25 @@ __device__ __forceinline__ float div_const(float a, float d, float r, int fast) 
     return __fdiv_rn(a, d);
 }
 
+// a / d for any a, for sweeps whose values lie below the verified range (a crystal at 0 C): a division
+// of denormals takes some hundred instructions, and a block that meets them holds up its whole
+// launch. Numerators below 2^-100 are divided 2^64 times larger, where the corrected product is
+// verified (for d in [2^-20, 2^20), see verify_fast_division); scaling the quotient back rounds
+// again only where it is denormal, and rounds wrongly only if the first rounding ended half way
+// between two denormals, from where the sign of the residual tells the way.
+inline __device__ __noinline__ float div_ieee(float a, float d) { return __fdiv_rn(a, d); }
+__device__ __forceinline__ float div_any(float a, float d, float r, int fast) {
+    const float m = fabsf(a);
+    if (!(fast && m < 0x1p101f && (m >= 0x1p-100f || (d >= 0x1p-20f && d < 0x1p20f)))) return div_ieee(a, d);
+    const bool tiny = m < 0x1p-100f;
+    const float x = tiny ? a * 0x1p64f : a;
+    const float q0 = x * r, q = fmaf(fmaf(-q0, d, x), r, q0);
+    if (!tiny) return q;
+    const float t = q * 0x1p-64f, diff = fmaf(-0x1p64f, t, q), rem = fmaf(-q, d, x);
+    const bool past = fabsf(diff) == 0x1p-86f && rem != 0.0f && (rem > 0.0f) == (diff > 0.0f);
+    return past ? t + copysignf(0x1p-149f, diff) : m > 0.0f ? t : a;
+}
+
 // (float)(((double)s + K) * (double)D), the edge formulas' last step (Tfield.h:162-195), with
 // K = kh + kl to 48 bits. The sum and product are carried as pairs of floats, which is within
 // 2^-44 (|s| + |K|) |D| of the exact value, as the double result is; where the float roundings of both
