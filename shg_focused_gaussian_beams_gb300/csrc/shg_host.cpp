@@ -98,9 +98,10 @@ float crystal_index(int crystal, float L, float T) {
 // Scales of the marched fields (shg_march.cuh): they make both coupling constants of dA/dz equal
 // to 1. Without coupling (d_eff = 0, or below 1e-12 pm/V, where kp < 2^-60 and p^2 would
 // underflow) the fields are held so small that the products vanish against them and p^2 is zero:
-// the fields diffract and are absorbed, and an SH that starts at zero stays zero.
+// the fields diffract and are absorbed, and an SH that starts at zero stays zero. A coupling that is
+// not a number is one: its scales, and with them the fields, are NaN.
 static void march_scales(InstDesc &d) {
-    const bool coupled = std::fabs(d.kp) >= 0x1p-60f && std::fabs(d.ks) >= 0x1p-60f;
+    const bool coupled = !(std::fabs(d.kp) < 0x1p-60f || std::fabs(d.ks) < 0x1p-60f);
     d.ss = coupled ? d.kp : 0x1p-60f;
     d.sp = coupled ? sqrtf(d.kp * d.ks) : 0x1p-100f;
     d.isp = 1.0f / d.sp;
