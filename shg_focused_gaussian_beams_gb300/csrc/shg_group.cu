@@ -18,6 +18,7 @@
 
 #include "shg_internal.h"
 #include "shg_coop.cuh"
+#include "shg_group_queue.cuh"
 #include "shg_stream.cuh"
 
 namespace shg {
@@ -66,16 +67,18 @@ __global__ void __launch_bounds__(GroupShape<N>::TPB, N >= 128 ? 2 : 3)
         target += BPI;
         return grid_barrier(bar, target, err);
     };
-    for (;;) {
-        // the group's first block takes the next solve; the others read it after the barrier (it
-        // is written again only after a later barrier of this solve's march)
+    auto take = [&] {
         if (rank == 0 && tid == 0) *(volatile unsigned *)slot = atomicAdd(words, 1u);
-        if (!meet()) return;
-        const unsigned job = ld_acquire_gpu(slot);
-        if (job >= (unsigned)njobs) return;
+    };
+    auto read = [&] { return ld_acquire_gpu(slot); };
+    // a bad descriptor skips the solve
+    auto good = [&](unsigned j) {
+        const InstDesc &d = inst[list[j]];
+        return SHG_REQUIRE(d.n == N && d.nsteps < d.nz && d.nsteps >= 1, kChkDescriptor, j);
+    };
+    unsigned job;
+    while (group_next(job, (unsigned)njobs, take, meet, read, good)) {
         const InstDesc &d = inst[list[job]];
-        // a bad descriptor skips the solve in every block of the group alike
-        if (!SHG_REQUIRE(d.n == N && d.nsteps < d.nz && d.nsteps >= 1, kChkDescriptor, job)) continue;
         const int K = d.nsteps;
         for (int s = 0; s <= K; ++s) {
             rows_body<N, true>(d, rank * LPB + tid / G, tid % G, s, scr + (tid / G) * LineScratch<N, G>::SIZE, tws);
