@@ -266,6 +266,13 @@ int shg_check_status(int *enabled, int *site, long long *value);
 /* Check build only: a kernel that touches no memory records (site 1, value), showing that a
  * failure reaches shg_check_status. SHG_ERR_UNSUPPORTED in other builds. */
 int shg_check_selftest(long long value);
+/* Every build: `launches` launches of the blocked heat sweep (`levels` = 1 or 2 sweeps each)
+ * in a given tiling, for tests of what the planner chooses on other grids: 256 or 512 threads a
+ * block, regions of vx (a power of two, 2 to 32) four-column vectors a row, chunks of zc planes.
+ * Buffers as for shg_heat_sweeps_device, 16-byte aligned; the result is in Ta for an even number
+ * of launches, in Tb for an odd one. SHG_ERR_INVALID for what is no tiling of the grid. */
+int shg_check_heat_tiling(const shg_config *cfg, void *Ta, void *Tb, const void *QK, float t_inf, int launches, int bc,
+                          int levels, int threads, int vx, int zc, void *stream);
 
 /* ---- Batched gradient of the THERMAL z-march (fixed temperature fields) ----------- */
 /* No counterpart in the reference (its THERMAL Solver::run, Solver.h:287-340, is forward

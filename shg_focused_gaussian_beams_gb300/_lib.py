@@ -99,6 +99,7 @@ SIGNATURES = {
     "shg_thgrad_device_bytes": (C.c_double, [_vp]),
     "shg_check_status": (_i, [_pi, _pi, C.POINTER(C.c_longlong)]),
     "shg_check_selftest": (_i, [C.c_longlong]),
+    "shg_check_heat_tiling": (_i, [C.POINTER(Config), _vp, _vp, _vp, _f, _i, _i, _i, _i, _i, _i, _vp]),
 }
 
 _lib = None

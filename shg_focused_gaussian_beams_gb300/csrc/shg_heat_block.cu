@@ -269,6 +269,8 @@ __device__ __forceinline__ int heat_chunk(float *__restrict__ Tf, const float *_
     const int v = threadIdx.x & (vx - 1), r = R * (threadIdx.x / vx);
     const int x = (int)blockIdx.x * g.txi - g.xh + 4 * v, y = (int)blockIdx.y * g.tyi - g.yh + r;
     const size_t sxy = (size_t)g.nx * g.ny;
+    // a shared plane holds the region's rows, and the grid a vector at least (block-uniform)
+    if (!SHG_REQUIRE(rows * row == PL && (vx & (vx - 1)) == 0 && g.nx % 4 == 0 && g.nx >= 8, kChkHeatVoxel, vx)) return z1;
     // this thread's first vector in shared plane 0, and the rows above and below its own;
     // planes: input ring, Q/k ring, levels 1..K-1
     float *const sm = hb_smem + (r * vx + v) * 4, *const sm1 = sm + row;
@@ -301,13 +303,14 @@ __device__ __forceinline__ int heat_chunk(float *__restrict__ Tf, const float *_
     const int dy1 = (yc1 - yc0) * g.nx;
     const float *srcT = Ti + plo * sxy + yc0 * g.nx + xc, *srcQ = QK + plo * sxy + yc0 * g.nx + xc;
     float *dst = Tf + z0 * sxy + yc0 * g.nx + xc;
+    auto held = [&](long long o) { return SHG_REQUIRE(o >= 0 && o + 3 < (long long)(sxy * g.nz), kChkHeatVoxel, o); };
     auto fetch = [&](int slot) {  // plane fp, and Q/k of plane fp - 1 (first used when plane fp has arrived)
         if (fp < pin) {
-            cp_async16(sm + slot * PL, srcT, in[0]);
-            cp_async16(sm1 + slot * PL, srcT + dy1, in[1]);
+            cp_async16(sm + slot * PL, srcT, in[0] && held(srcT - Ti));
+            cp_async16(sm1 + slot * PL, srcT + dy1, in[1] && held(srcT + dy1 - Ti));
             if (fp > plo) {
-                cp_async16(sm + (kRing + slot) * PL, srcQ, in[0]);
-                cp_async16(sm1 + (kRing + slot) * PL, srcQ + dy1, in[1]);
+                cp_async16(sm + (kRing + slot) * PL, srcQ, in[0] && held(srcQ - QK));
+                cp_async16(sm1 + (kRing + slot) * PL, srcQ + dy1, in[1] && held(srcQ + dy1 - QK));
                 srcQ += sxy;
             }
             srcT += sxy;
@@ -597,6 +600,29 @@ bool heat_block_supported(int nx, int ny, int nz) {
 // (47 us is the HBM copy rate for one sweep's 12 bytes per voxel.) At 256x256x400 with two
 // sweeps per launch: 79 warp instructions per four voxels and level of a warp, 51 % issue, FMA
 // pipe 23 % (the packed forms take it for two cycles), shared-memory latency the top stall.
+// The plan of one tiling: regions of vx vectors by kRows threads / vx rows (a whole row, or tiles with a
+// halo vector on each side), chunks of zc planes. False for what is none.
+static bool tile_plan(int nx, int ny, int nz, int levels, int threads, int vx, int zc, HeatBlockPlan *out) {
+    if (levels < 1 || levels > kMaxLevels || (threads != 256 && threads != 512) || vx < 2 || vx > 32 || (vx & (vx - 1)) ||
+        zc < 1 || zc > nz)
+        return false;
+    const int vecs = nx / 4, rows = kRows * (threads / vx);
+    const bool whole_x = vx >= vecs, whole_y = rows >= ny;
+    if ((!whole_x && vx < 8) || (!whole_y && rows <= 2 * levels)) return false;
+    const int ti = whole_x ? vecs : vx - 2, tyi = whole_y ? ny : rows - 2 * levels;
+    out->g = HeatBlockGrid{nx, ny, nz, vx, 4 * ti, tyi, whole_x ? 0 : 4, whole_y ? 0 : levels, zc};
+    out->grid = dim3((vecs + ti - 1) / ti, (ny + tyi - 1) / tyi, (nz + zc - 1) / zc);
+    out->threads = threads;
+    out->levels = levels;
+    out->smem = (size_t)shared_planes(levels) * plane_floats(threads, kRows) * sizeof(float);
+    return true;
+}
+
+static cudaError_t allow_shared(const HeatBlockPlan &p, int bc) {
+    return cudaFuncSetAttribute(kernel_of(bc, p.levels, p.threads), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)p.smem);
+}
+
 static cudaError_t search_plan(int dev, int nx, int ny, int nz, int bc, int levels, HeatBlockPlan *out) {
     int sms = 0;
     cudaError_t e;
@@ -608,15 +634,10 @@ static cudaError_t search_plan(int dev, int nx, int ny, int nz, int bc, int leve
     for (int K = levels ? levels : 1; K <= (levels ? levels : kMaxLevels); ++K)
         for (int threads = 256; threads <= 512; threads *= 2)
             for (int vx = 2; vx <= 32; vx *= 2) {
-                // region rows of vx vectors: the whole row, or tiles with a halo vector on each side
-                const bool whole_x = vx >= vecs;
-                const int rows = kRows * (threads / vx);
-                const bool whole_y = rows >= ny;
-                if ((!whole_x && vx < 8) || (!whole_y && rows <= 2 * K)) continue;
-                const int ti = whole_x ? vecs : vx - 2, tx = (vecs + ti - 1) / ti;
-                const int tyi = whole_y ? ny : rows - 2 * K, ty = (ny + tyi - 1) / tyi;
+                HeatBlockPlan t;
+                if (!tile_plan(nx, ny, nz, K, threads, vx, nz, &t)) continue;
                 const int bps = 512 / threads, warps = threads / 128;  // blocks per SM, warps per scheduler of one
-                const long long slots = (long long)bps * sms, tiles = (long long)tx * ty;
+                const long long slots = (long long)bps * sms, tiles = (long long)t.grid.x * t.grid.y;
                 for (int nc = 1; nc <= nz; ++nc) {
                     const int zc = (nz + nc - 1) / nc;
                     const long long blocks = tiles * ((nz + zc - 1) / zc), waves = (blocks + slots - 1) / slots;
@@ -627,19 +648,19 @@ static cudaError_t search_plan(int dev, int nx, int ny, int nz, int bc, int leve
                     if (bytes > kL2) cost = std::max(cost, bytes / kBytesPerCycle);
                     if (cost / K < best) {
                         best = cost / K;
-                        out->g = HeatBlockGrid{nx, ny, nz, vx, 4 * ti, tyi, whole_x ? 0 : 4, whole_y ? 0 : K, zc};
-                        out->grid = dim3(tx, ty, (nz + zc - 1) / zc);
-                        out->threads = threads;
-                        out->levels = K;
+                        tile_plan(nx, ny, nz, K, threads, vx, zc, out);
                     }
                     if (blocks > 8 * slots) break;
                 }
-                if (whole_x) break;
+                if (vx >= vecs) break;
             }
     if (best == 1e300) return cudaErrorInvalidConfiguration;
-    out->smem = (size_t)shared_planes(out->levels) * plane_floats(out->threads, kRows) * sizeof(float);
-    return cudaFuncSetAttribute(kernel_of(bc, out->levels, out->threads), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)out->smem);
+    return allow_shared(*out, bc);
+}
+
+cudaError_t heat_block_tiling(int nx, int ny, int nz, int bc, int levels, int threads, int vx, int zc, HeatBlockPlan *out) {
+    if (!heat_block_supported(nx, ny, nz) || !tile_plan(nx, ny, nz, levels, threads, vx, zc, out)) return cudaErrorInvalidValue;
+    return allow_shared(*out, bc);
 }
 
 cudaError_t heat_block_plan(int nx, int ny, int nz, int bc, int levels, HeatBlockPlan *out) {

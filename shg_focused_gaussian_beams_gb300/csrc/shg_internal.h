@@ -106,6 +106,8 @@ cudaError_t verify_fast_division(float d, float r, unsigned long long *d_count, 
 struct HeatBlockPlan;
 bool heat_block_supported(int nx, int ny, int nz);
 cudaError_t heat_block_plan(int nx, int ny, int nz, int bc, int levels, HeatBlockPlan *out);
+// The plan of a given tiling (cudaErrorInvalidValue for what is none).
+cudaError_t heat_block_tiling(int nx, int ny, int nz, int bc, int levels, int threads, int vx, int zc, HeatBlockPlan *out);
 cudaError_t launch_heat_block(float *Tf, const float *Ti, const float *QK, const HeatCoef &c, int bc,
                               const HeatBlockPlan &p, cudaStream_t st);
 // shg_heat_tma.cu: the TMA-staged sweep (NX % 4 == 0) and its pipeline error word. Each

@@ -142,8 +142,9 @@ static int heat_levels_asked() {
 
 // `n` Jacobi sweeps on `st` between buf[0] and buf[1], starting from buf[cur], which is
 // updated to the buffer that holds the result. Grids whose rows are whole 16-byte vectors take
-// the blocked kernel (shg_heat_block.cu, one or two sweeps per launch); others, unaligned
-// buffers and a kernel selected by name take one launch of launch_heat per sweep. With
+// the blocked kernel (shg_heat_block.cu, one or two sweeps per launch); others and a kernel
+// selected by name take one launch of launch_heat per sweep (which refuses buffers of such grids
+// that are not 16-byte aligned, unless a kernel other than "tma" is named). With
 // `as_single` the buffers end as after n launches of one sweep: the result in buf[n & 1] (from
 // cur = 0), the state before the last sweep in the other.
 static int heat_sweeps_enqueue(float *const (&buf)[2], int &cur, const float *qk, const HeatCoef &hc, int nx, int ny,
@@ -546,6 +547,26 @@ int shg_heat_sweeps_device(const shg_config *cfg, void *Ta, void *Tb, const void
                                true, err, st));
     // heat_pipeline_ok synchronises `st` and clears the word before it returns to the pool
     return heat_pipeline_ok(err, st);
+}
+
+int shg_check_heat_tiling(const shg_config *cfg, void *Ta, void *Tb, const void *QK, float t_inf, int launches, int bc,
+                          int levels, int threads, int vx, int zc, void *stream) {
+    TH_TRY(thermal_component_cfg(cfg));
+    const uintptr_t a = reinterpret_cast<uintptr_t>(Ta), b = reinterpret_cast<uintptr_t>(Tb), q = reinterpret_cast<uintptr_t>(QK);
+    HeatBlockPlan p;
+    if (!a || !b || !q || ((a | b | q) & 15) || launches < 0 || (bc != 0 && bc != 1) ||
+        heat_block_tiling(cfg->nx, cfg->ny, cfg->nz, bc, levels, threads, vx, zc, &p) != cudaSuccess) {
+        set_error("shg_check_heat_tiling: null or unaligned buffer, or no tiling of this grid");
+        return SHG_ERR_INVALID;
+    }
+    HeatCoef hc = make_heat_coef(*cfg, t_inf);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    TH_TRY(enable_fast_division(hc, st));
+    float *const buf[2] = {static_cast<float *>(Ta), static_cast<float *>(Tb)};
+    for (int k = 0; k < launches; ++k)
+        TH_CUDA(launch_heat_block(buf[~k & 1], buf[k & 1], static_cast<const float *>(QK), hc, bc, p, st));
+    TH_CUDA(cudaStreamSynchronize(st));
+    return SHG_OK;
 }
 
 int shg_dk_thermal(const shg_config *cfg, const float *T, float *DK, float *NP, float *NS) {
