@@ -61,7 +61,11 @@ struct CoopShape {
     static constexpr int TC = 32 / G;                    // columns per column group
     static constexpr int ROW_UNITS = N / LPB;            // groups of LPB lines
     static constexpr int COL_UNITS = 2 * (N / TC);       // column groups of both fields
-    static constexpr bool SPLIT = RowLanes<N, true>::SPLIT;
+    // Columns of 16 x 8 points are split over two warps. Where both DFTs are of 16 points (N = 256) each warp of a
+    // pair needs all inputs of both and the pair's outputs besides, which costs more than the shorter chain gives:
+    // one 256 x 256 x 400 march 2.87 ms, split 3.16 (its THERMAL march in a run of two 12.7, 13.3); 128 x 128 x 200
+    // 1.19, split 1.10 (3.73, 3.53).
+    static constexpr bool SPLIT = RowLanes<N, true>::SPLIT && E != G;
     static constexpr int GW = SPLIT ? 2 : 1;             // warps of a column group
     static constexpr int OUT = E / GW;                   // spectrum values per thread
     static_assert(TC * G == 32, "a column group is one warp, two of split lanes");

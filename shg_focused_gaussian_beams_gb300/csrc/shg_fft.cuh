@@ -387,35 +387,26 @@ struct WarpSync {
 
 // One z step's column pass of a line on split lanes (t, h): backward transform of thread t's elements
 // v of the column, mid(r, value) on this lane's outputs (SplitLine::spec), forward transform to o
-// (SplitLine::nat). Column scratch: elements STRIDE apart.
+// (SplitLine::nat). Column scratch: elements STRIDE apart. Two DFTs per thread (Q = 2): a lane's outputs
+// of the first transform are its inputs of the second.
 template <int N, int STRIDE, bool TS, class Sync, class Mid>
 __device__ __forceinline__ void column_split(const float2 (&v)[N / LineShape<N>::G],
                                              float2 (&o)[N / LineShape<N>::G / 2], int t, int h, float2 *sc,
                                              const float2 *__restrict__ tab, Sync sync, Mid mid) {
     constexpr int G = LineShape<N>::G;
     using L = SplitLine<N, G>;
+    static_assert(L::Q == 2 && L::IN == L::OUT, "split columns hold two DFTs per thread");
     fft_nat_to_spec_split<N, G, +1, STRIDE, G, TS>(v, o, t, h, sc, tab, sync);
-#pragma unroll
-    for (int r = 0; r < L::OUT; ++r) o[r] = mid(r, o[r]);
     float2 w[L::IN];
-    if constexpr (L::Q == 1) {  // the pair's lanes exchange their outputs
-        sync();
 #pragma unroll
-        for (int r = 0; r < L::OUT; ++r) sc[(t * G + 2 * r + h) * STRIDE] = o[r];
-        sync();
-#pragma unroll
-        for (int r = 0; r < L::IN; ++r) w[r] = sc[(t * G + r) * STRIDE];
-    } else {
-#pragma unroll
-        for (int r = 0; r < L::OUT; ++r) w[r] = o[r];
-    }
+    for (int r = 0; r < L::OUT; ++r) w[r] = mid(r, o[r]);
     fft_spec_to_nat_split<N, G, -1, STRIDE, G, TS>(w, o, t, h, sc, tab, sync);
 }
 
 // Row transforms of a line by LW consecutive lanes of a warp, between a row in memory (natural
 // frequency order) and the line buffer in shared memory (natural order). Lines of 16-point DFTs
 // (N >= 128) are split; 8-point ones save no more than the pairs' doubled loads cost (one 64 x 64
-// solve on the persistent grid 1105 us, split 1112; 256 x 256: 2.89 ms, split 2.63).
+// solve on the persistent grid 1105 us, split 1112; 256 x 256 by the streaming passes: 2.89 ms, split 2.63).
 template <int N, bool TS>
 struct RowLanes {
     static constexpr int G = LineShape<N>::G, E = N / G;
@@ -503,23 +494,18 @@ __device__ __forceinline__ void hprop_load(const float2 *__restrict__ H, int x, 
     }
 }
 
-// The propagator values of split lane (t, h)'s outputs of column x.
+// The propagator values of split lane (t, h)'s outputs of column x: registers h G + r, words h G / 2 + r / 2.
 template <int N>
 __device__ __forceinline__ void split_hprop_load(const float2 *__restrict__ H, int x, int t, int h,
                                                  float2 (&o)[N / LineShape<N>::G / 2]) {
     constexpr int G = LineShape<N>::G, E = N / G;
-    if constexpr (E == G) {  // register 2 r + h: half h of word r
+    static_assert(SplitLine<N, G>::Q == 2, "split columns hold two DFTs per thread");
+    const float4 *p = reinterpret_cast<const float4 *>(H);
 #pragma unroll
-        for (int r = 0; r < E / 2; ++r)
-            o[r] = __ldg(&SHG_AT(H, (((size_t)t * (E / 2) + r) * N + x) * 2 + h, (size_t)N * N, kChkPropagator));
-    } else {  // registers h G + r: words h G / 2 + r / 2
-        const float4 *p = reinterpret_cast<const float4 *>(H);
-#pragma unroll
-        for (int r = 0; r < G / 2; ++r) {
-            const float4 q = __ldg(&SHG_AT(p, ((size_t)t * (E / 2) + h * (G / 2) + r) * N + x, (size_t)N * N / 2, kChkPropagator));
-            o[2 * r] = make_float2(q.x, q.y);
-            o[2 * r + 1] = make_float2(q.z, q.w);
-        }
+    for (int r = 0; r < G / 2; ++r) {
+        const float4 q = __ldg(&SHG_AT(p, ((size_t)t * (E / 2) + h * (G / 2) + r) * N + x, (size_t)N * N / 2, kChkPropagator));
+        o[2 * r] = make_float2(q.x, q.y);
+        o[2 * r + 1] = make_float2(q.z, q.w);
     }
 }
 
