@@ -204,8 +204,7 @@ __device__ __forceinline__ void rows_pt_body(const InstDesc &d, int line0, int s
         block_add_double((double)vp.x * vp.x + (double)vp.y * vp.y, d.acc + 2);
         return;
     }
-    march_turn(vs, turn);
-    rk4_march(vp, vs, d);
+    rk4_turned(vp, vs, turn, d);
     *pP = vp;
     *pS = vs;
     __syncthreads();
