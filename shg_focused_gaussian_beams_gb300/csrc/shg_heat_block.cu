@@ -533,19 +533,6 @@ __device__ __forceinline__ int heat_chunk(float *__restrict__ Tf, const float *_
     }
 }
 
-// The planes from a value out of range on. A crystal at 0 C has them: it holds zeros for good on the
-// faces that are never written, and heat spreads into the rest in small values. us per sweep with heat
-// down to 1e-20 from a zero crystal, open top / oven, ordinary temperatures in brackets: 64x64x200 8.1 (5.2)
-// / 5.9 (3.9), 256x256x400 83 (60) / 57 (46); with the heat of a Gaussian that underflows to denormals
-// 8.4 / 6.4, 128x128x200 19 (8.8) / 13 (6.3), 256x256x400 227 / 181, where a launch waits for its blocks
-// in the corners (the single-sweep kernels: 17 / 11, 23 / 16, 95 / 83). Out of line, so that it takes no
-// registers from the ordinary chunk (in line 64x64x200 open top 5.4 -> 5.5, out of line 5.2).
-template <int BC, int K, int THREADS>
-__device__ __noinline__ void heat_chunk_any(float *Tf, const float *Ti, const float *QK, const HeatCoef &c,
-                                            const HeatBlockGrid &g, int z0, int z1) {
-    heat_chunk<BC, K, THREADS, false>(Tf, Ti, QK, c, g, z0, z1);
-}
-
 template <int BC, int K, int THREADS>
 __global__ void __launch_bounds__(THREADS, 512 / THREADS)
     k_heat_block(float *__restrict__ Tf, const float *__restrict__ Ti, const float *__restrict__ QK,
@@ -556,7 +543,15 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS)
     if (g.zc <= 16) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int z0 = (int)blockIdx.z * g.zc, z1 = min(g.nz, z0 + g.zc);
     const int z = heat_chunk<BC, K, THREADS, true>(Tf, Ti, QK, c, g, z0, z1);
-    if (z < z1) heat_chunk_any<BC, K, THREADS>(Tf, Ti, QK, c, g, z, z1);
+    // The planes from a value out of range on. A crystal at 0 C has them: it holds zeros for good on the
+    // faces that are never written, and heat spreads into the rest in small values. us per sweep with
+    // heat down to 1e-20 from a zero crystal, open top / oven, ordinary temperatures in brackets:
+    // 64x64x200 8.2 (5.1) / 5.4 (3.8), 128x128x200 11.8 (8.8) / 7.8 (6.3), 256x256x400 74 (60) / 52 (45.6). With
+    // the heat of a Gaussian that underflows to denormals a launch waits for its blocks in the corners:
+    // 64x64x200 8.4 / 6.0, 128x128x200 19 / 13, 256x256x400 265 / 215 (the single-sweep kernels: 17 / 11, 23 / 16,
+    // 95 / 83). In line: as a function called here it cost the ordinary chunk registers that are kept
+    // across calls (256x256x400 oven 45.9; 77 / 56 from a zero crystal, 274 / 233 with denormals).
+    if (z < z1) heat_chunk<BC, K, THREADS, false>(Tf, Ti, QK, c, g, z, z1);
 }
 
 typedef void (*HeatBlockKernel)(float *, const float *, const float *, const HeatCoef, const HeatBlockGrid);
