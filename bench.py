@@ -536,6 +536,56 @@ def per_instance_rate(sample, device):
                     "synchronised), handles created and warmed outside the timed region"}
 
 
+# the whole march of a class in one kernel: persistent groups of blocks, clusters, the cooperative grid
+ONE_LAUNCH = ("group<", "resident<", "cluster<", "coop<")
+
+
+def sweep_roofline(prof, insts, sms, sm_mhz):
+    """Roofline of the kernel with the largest share of a profiled run (name -> launches, ms, algorithmic
+    bytes). The fraction of the HBM copy rate stands at the top level; a march in one kernel keeps its
+    fields on chip (L2 or shared memory), where `bound` is instruction issue if that is nearer its peak."""
+    dom = max(prof, key=lambda k: prof[k][1])
+    n_l, ms_k, bytes_k = prof[dom]
+    n_dom = int(dom[dom.index("<") + 1:-1]) if "<" in dom else 0
+    pt_rate = bytes_k / 32.0 / (ms_k * 1e-3)  # grid-pt.z-steps/s of a march in one kernel
+    peak, peak_kind = measured_hbm()
+    achieved = bytes_k / (ms_k * 1e-3) / 1e9
+    tr = ncu_traffic(dom)
+    traffic = None
+    if tr and "bytes_per_solve" in tr and dom.startswith(ONE_LAUNCH):
+        # each solve's fields move in and out once (and its propagators, where they are read from
+        # L2): traffic scales with the solves of the launch, not the steps
+        traffic = tr["bytes_per_solve"] * sum(1 for i in insts if i.nx == n_dom)
+    elif tr and "bytes_per_point" in tr:
+        traffic = tr["bytes_per_point"] * bytes_k / n_l / (32.0 if dom.startswith("rows") else 48.0)
+    issue = fp32 = None
+    if tr and "thread_inst_per_pt_step" in tr:
+        # thread-instructions per second (ncu count per pt.step x the launch's pt.steps from
+        # its algorithmic bytes, 32 B per pt.step) against the issue peak of 4 schedulers x
+        # 32 lanes per SM at the sampled SM clock
+        inst_s = tr["thread_inst_per_pt_step"] * pt_rate
+        peak_inst = sms * 128 * sm_mhz * 1e6
+        issue = {"achieved": inst_s, "peak": peak_inst, "unit": "thread-instructions/s", "frac": inst_s / peak_inst,
+                 "thread_inst_per_pt_step": tr["thread_inst_per_pt_step"], "source": tr.get("inst_source"),
+                 "peak_note": f"{sms} SMs x 128 lanes x {sm_mhz:.0f} MHz (nominal issue rate)"}
+    if dom.startswith(ONE_LAUNCH):
+        # flops of the method per grid-pt.z-step: 4 2D FFTs at 5 N log2 N, 2 propagator
+        # products, 2 RK4 calls (20 log2(N^2) + 456; sincos not counted), against the nominal
+        # FP32 rate (no measured FP32 peak exists): SMs x 128 lanes x 2 flop x SM clock
+        flop_pt = 20.0 * math.log2(n_dom * n_dom) + 456.0
+        fl_s = flop_pt * pt_rate
+        peak_fl = sms * 128 * 2 * sm_mhz * 1e6
+        fp32 = {"achieved": fl_s / 1e12, "peak": peak_fl / 1e12, "unit": "TFLOP/s", "frac": fl_s / peak_fl,
+                "flop_per_pt_step": flop_pt, "peak_note": "nominal FP32 rate at the sampled SM clock"}
+    frac = achieved / peak
+    return {"bound": "issue" if issue and issue["frac"] > frac else "hbm", "kernel": dom, "achieved": achieved,
+            "peak": peak, "unit": "GB/s", "frac": frac, "peak_source": peak_kind, "launches": n_l, "issue": issue,
+            "fp32": fp32, "ms_per_launch": ms_k / n_l, "algorithmic_bytes_per_launch": bytes_k / n_l,
+            "traffic": traffic, "traffic_source": None if tr is None else tr.get("source"),
+            "share_of_step": ms_k / sum(v[1] for v in prof.values()),
+            "kernels": {k: {"launches": v[0], "ms": v[1], "GBps": v[2] / (v[1] * 1e-3) / 1e9} for k, v in prof.items()}}
+
+
 def run_ours(args):
     import torch
     from shg_focused_gaussian_beams_gb300.solver import Sweep
@@ -601,55 +651,8 @@ def run_ours(args):
     per = per_instance_rate(insts[:64], local) if rank == 0 else None
 
     # roofline of the dominant kernel from an instrumented run (per-launch CUDA events)
-    prof = sw.profile()
-    dom = max(prof, key=lambda k: prof[k][1])
-    n_l, ms_k, bytes_k = prof[dom]
-    peak, peak_kind = measured_hbm()
-    achieved = bytes_k / (ms_k * 1e-3) / 1e9
-    tr = ncu_traffic(dom)
-    traffic = None
-    if tr and "bytes_per_solve" in tr and dom.startswith("resident<"):
-        # the resident march moves each solve's fields in and out once (and reads its
-        # propagators from L2): traffic scales with the solves of the launch, not the steps
-        n_dom = int(dom[len("resident<"):-1])
-        traffic = tr["bytes_per_solve"] * sum(1 for i in insts if i.nx == n_dom)
-    elif tr and "bytes_per_point" in tr:
-        traffic = tr["bytes_per_point"] * bytes_k / n_l / (32.0 if dom.startswith("rows") else 48.0)
-    issue = None
-    if tr and "thread_inst_per_pt_step" in tr:
-        # the resident march keeps its fields on chip, so its bound is FP32 instruction issue:
-        # thread-instructions per second (ncu count per pt.step x the launch's pt.steps from
-        # its algorithmic bytes, 32 B per pt.step) against the issue peak of 4 schedulers x
-        # 32 lanes per SM at the sampled SM clock
-        props = torch.cuda.get_device_properties(local)
-        pt_steps = bytes_k / n_l / 32.0
-        inst_s = tr["thread_inst_per_pt_step"] * pt_steps / (ms_k / n_l * 1e-3)
-        sm_mhz = clk.summary().get("sm_mhz") or 2070.0
-        peak_inst = props.multi_processor_count * 128 * sm_mhz * 1e6
-        issue = {"achieved": inst_s, "peak": peak_inst, "unit": "thread-instructions/s", "frac": inst_s / peak_inst,
-                 "thread_inst_per_pt_step": tr["thread_inst_per_pt_step"], "source": tr.get("inst_source"),
-                 "peak_note": f"{props.multi_processor_count} SMs x 128 lanes x {sm_mhz:.0f} MHz (nominal issue rate)"}
-    fp32 = None
-    if dom.startswith(("resident<", "cluster<", "coop<")):  # the whole march in one kernel
-        # flops of the method per grid-pt.z-step: 4 2D FFTs at 5 N log2 N, 2 propagator
-        # products, 2 RK4 calls (20 log2(N^2) + 456; sincos not counted), against the nominal
-        # FP32 rate (no measured FP32 peak exists): SMs x 128 lanes x 2 flop x SM clock
-        props = torch.cuda.get_device_properties(local)
-        n_dom = int(dom[dom.index("<") + 1:-1])
-        flop_pt = 20.0 * math.log2(n_dom * n_dom) + 456.0
-        pt_steps = bytes_k / n_l / 32.0
-        fl_s = flop_pt * pt_steps / (ms_k / n_l * 1e-3)
-        sm_mhz = clk.summary().get("sm_mhz") or 2070.0
-        peak_fl = props.multi_processor_count * 128 * 2 * sm_mhz * 1e6
-        fp32 = {"achieved": fl_s / 1e12, "peak": peak_fl / 1e12, "unit": "TFLOP/s", "frac": fl_s / peak_fl,
-                "flop_per_pt_step": flop_pt, "peak_note": "nominal FP32 rate at the sampled SM clock"}
-    roof = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak, "peak_source": peak_kind, "launches": n_l, "issue": issue, "fp32": fp32,
-            "ms_per_launch": ms_k / n_l, "algorithmic_bytes_per_launch": bytes_k / n_l,
-            "traffic": traffic,
-            "traffic_source": None if tr is None else tr.get("source"),
-            "share_of_step": ms_k / sum(v[1] for v in prof.values()),
-            "kernels": {k: {"launches": v[0], "ms": v[1], "GBps": v[2] / (v[1] * 1e-3) / 1e9} for k, v in prof.items()}}
+    roof = sweep_roofline(sw.profile(), insts, torch.cuda.get_device_properties(local).multi_processor_count,
+                          clk.summary().get("sm_mhz") or 2070.0)
 
     if rank == 0:
         cores = os.cpu_count() or 1
