@@ -15,7 +15,7 @@
 //
 // Why this split: the single-sweep kernel issues 77 thread instructions per voxel (seven shared
 // loads among them) at 80 % issue, above its memory time; four columns per thread and packed
-// arithmetic take 20. What each kernel measured, and when two sweeps per launch pay, stands at
+// arithmetic take 18. What each kernel measured, and when two sweeps per launch pay, stands at
 // heat_block_plan.
 #include <cuda_runtime.h>
 
@@ -592,9 +592,10 @@ bool heat_block_supported(int nx, int ny, int nz) {
 //   128x128x200 open top 21.0 -> 9.6 / 9.8,   oven 14.8 -> 7.6 / 6.7
 //   200x200x150 open top 32.5 -> 19.5 / 19.4, oven 25.4 -> 16.6 / 14.2
 //   256x256x400 open top 86.2 -> 69.2 / 65.9, oven 71.4 -> 64.8 / 48.4
-// (47 us is the HBM copy rate for one sweep's 12 bytes per voxel.) At 256x256x400 with two
-// sweeps per launch: 79 warp instructions per four voxels and level of a warp, 51 % issue, FMA
-// pipe 23 % (the packed forms take it for two cycles), shared-memory latency the top stall.
+// (47 us is the HBM copy rate for one sweep's 12 bytes per voxel.) The plan's choice now, same grids, open top /
+// oven: 3.9 / 2.3, 5.1 / 3.8, 4.4 / 3.6, 8.8 / 6.3, 17.8 / 13.3, 59.7 / 45.6. At 256x256x400 oven with two sweeps
+// per launch: 73 warp instructions per four voxels and level of a warp, 46 % issue, FMA pipe 22 % (the packed
+// forms take it for two cycles), shared-memory latency the top stall.
 // The plan of one tiling: regions of vx vectors by kRows threads / vx rows (a whole row, or tiles with a
 // halo vector on each side), chunks of zc planes. False for what is none.
 static bool tile_plan(int nx, int ny, int nz, int levels, int threads, int vx, int zc, HeatBlockPlan *out) {
