@@ -165,7 +165,8 @@ __global__ void __launch_bounds__(CptShape<N, CS>::TPB, 1)
                     aS += (double)q.x * q.x + (double)q.y * q.y;
                     aP += (double)p.x * p.x + (double)p.y * p.y;
                 } else {
-                    rk4_turned(p, q, ccur, d);
+                    march_turn(q, ccur);
+                    rk4_march(p, q, d);
                     sP[i] = p;
                     sS[i] = q;
                 }

@@ -204,7 +204,8 @@ __device__ __forceinline__ void rows_pt_body(const InstDesc &d, int line0, int s
         block_add_double((double)vp.x * vp.x + (double)vp.y * vp.y, d.acc + 2);
         return;
     }
-    rk4_turned(vp, vs, turn, d);
+    march_turn(vs, turn);
+    rk4_march(vp, vs, d);
     *pP = vp;
     *pS = vs;
     __syncthreads();

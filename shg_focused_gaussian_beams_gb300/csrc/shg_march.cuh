@@ -81,20 +81,26 @@ __device__ __forceinline__ void dads_point(float2 p, float2 s, float hp, float t
     ds.y = fmaf(p.x, p.x, fmaf(-p.y, p.y, -ny));
 }
 
-// Fields into the frame of slice 0 (z = 0), and back from the frame of c's slice.
+// Fields into the frame of slice 0 (z = 0), from slice s-1's to slice s's (c = stepc[s]; written as
+// s + (cos d - 1) s + ..., whose rounding is not biased the way a rounded cos d near 1 is), and
+// back from the frame of c's slice.
 __device__ __forceinline__ void march_enter(float2 &p, float2 &s, const InstDesc &d) {
     p = make_float2(d.sp * p.x, d.sp * p.y);
     s = make_float2(d.ss * s.x, d.ss * s.y);
+}
+__device__ __forceinline__ void march_turn(float2 &s, float4 c) {
+    s = make_float2(fmaf(c.y, s.y, fmaf(c.x, s.x, s.x)), fmaf(-c.y, s.x, fmaf(c.x, s.y, s.y)));
 }
 __device__ __forceinline__ void march_leave(float2 &p, float2 &s, float4 c, const InstDesc &d) {
     p = make_float2(d.isp * p.x, d.isp * p.y);
     s = make_float2(d.iss * fmaf(c.z, s.x, -c.w * s.y), d.iss * fmaf(c.z, s.y, c.w * s.x));
 }
 
-// The slopes k1 + 2 k2 + 2 k3 + k4 of one solverRK4 call (Solver.h:193-233, plain branch) in the march's
-// frame: stage offsets 0.5, 0.5, 1 without a dz factor; every stage uses the same z.
-__device__ __forceinline__ void rk4_slopes(float2 P, float2 S, const InstDesc &d, float2 &accp, float2 &accs) {
-    float2 kp, ks, ap, as;
+// One solverRK4 call (Solver.h:193-233, plain branch) in the march's frame: stage offsets 0.5,
+// 0.5, 1 without a dz factor, and the update A + (k1 + 2 k2 + 2 k3 + k4) dz/6; every stage uses
+// the same z.
+__device__ __forceinline__ void rk4_march(float2 &P, float2 &S, const InstDesc &d) {
+    float2 kp, ks, ap, as, accp, accs;
     dads_point(P, S, d.hp, d.tpa0, d.tpa1s, kp, ks);
     accp = kp;
     accs = ks;
@@ -113,28 +119,8 @@ __device__ __forceinline__ void rk4_slopes(float2 P, float2 S, const InstDesc &d
     dads_point(ap, as, d.hp, d.tpa0, d.tpa1s, kp, ks);
     accp = c_add(accp, kp);
     accs = c_add(accs, ks);
-}
-
-// One solverRK4 call: A + slopes dz/6.
-__device__ __forceinline__ void rk4_march(float2 &P, float2 &S, const InstDesc &d) {
-    float2 accp, accs;
-    rk4_slopes(P, S, d, accp, accs);
     P = make_float2(fmaf(accp.x, d.dz6, P.x), fmaf(accp.y, d.dz6, P.y));
     S = make_float2(fmaf(accs.x, d.dz6, S.x), fmaf(accs.y, d.dz6, S.y));
-}
-
-// From slice s-1's frame to slice s's (c = stepc[s]), then slice s's first call. The turn adds
-// t = (cos d - 1) s + ... to s; the call's slopes are those at s + t, and t and the call's increment go
-// to s together, so that a slice rounds the SH twice, once per call, as on fields that do not turn.
-// (With the turn rounded on its own, points without diffraction were 1.10 to 1.31 times as far from 64 bits
-// as by the fields themselves; now 0.99 to 1.06 times.) Four more instructions per point and z step; the 128 x 128
-// march by groups loses its spills: the 512-solve sweep 69.1 -> 66.7 ms, lone solves within 0.5 %.
-__device__ __forceinline__ void rk4_turned(float2 &P, float2 &S, float4 c, const InstDesc &d) {
-    const float2 t = make_float2(fmaf(c.y, S.y, c.x * S.x), fmaf(-c.y, S.x, c.x * S.y));
-    float2 accp, accs;
-    rk4_slopes(P, c_add(S, t), d, accp, accs);
-    P = make_float2(fmaf(accp.x, d.dz6, P.x), fmaf(accp.y, d.dz6, P.y));
-    S = make_float2(S.x + fmaf(accs.x, d.dz6, t.x), S.y + fmaf(accs.y, d.dz6, t.y));
 }
 
 // The same call on the fields themselves, with the slice's coupling constants c (the adjoint's

@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(ResShape<N, CS_, MINB_, G_>::THREADS, MINB_)
                     } else {
 #pragma unroll
                         for (int r = 0; r < E; ++r) {
-                            rk4_turned(vp[r], vs[r], ccur, d);
+                            march_turn(vs[r], ccur);
+                            rk4_march(vp[r], vs[r], d);
                         }
                         fft_spec_to_nat<N, G, +1, false, 1, G + 1, true>(vp, t, rsc, tab);
                         fft_spec_to_nat<N, G, +1, false, 1, G + 1, true>(vs, t, rsc, tab);

@@ -104,7 +104,8 @@ __device__ __forceinline__ void rows_body(const InstDesc &d, int line, int t, in
     const float4 c2 = d.stepc[s];
 #pragma unroll
     for (int r = 0; r < E; ++r) {
-        rk4_turned(vp[r], vs[r], c2, d);
+        march_turn(vs[r], c2);
+        rk4_march(vp[r], vs[r], d);
     }
     fft_spec_to_nat<N, G, +1, false, 1, G + 1, CG>(vp, t, sc, tab);
     fft_spec_to_nat<N, G, +1, false, 1, G + 1, CG>(vs, t, sc, tab);
