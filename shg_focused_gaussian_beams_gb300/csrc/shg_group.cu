@@ -12,8 +12,10 @@
 // solve on (13 % fewer instructions left its 256 x 256 class at 78 ms), and every SM holds
 // blocks, where sixteen-CTA clusters leave a quarter of the slots empty. Measured, 198 solves of
 // 256 x 256: streaming 75.8 ms, sixteen-CTA clusters 78.5, groups 52.8 (1.21 us per solve and z
-// step, 65 % of the FMA issue bound); 141 of 128 x 128: 13.4, 9.8, 9.4; 64 x 64 solves fit one CTA's
-// shared memory and stay there (3.4 ms against 6.2). The 512-solve sweep 85.2 -> 66.3 ms.
+// step); 141 of 128 x 128: 13.4, 9.8, 9.4; 64 x 64 solves fit one CTA's
+// shared memory and stay there (3.4 ms against 6.2). The 512-solve sweep 85.2 -> 66.3 ms. Its
+// 179 solves of 256 x 256 now: groups 47.3 ms, streaming 67.8, clusters 71.1; 406 instructions per grid point and z
+// step, 0.57 of the issue slots, the rest mostly barriers.
 #include <cuda_runtime.h>
 
 #include "shg_internal.h"
